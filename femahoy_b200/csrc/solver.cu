@@ -2057,7 +2057,7 @@ SolverImpl::~SolverImpl() {
 
 template <class T>
 size_t Hierarchy<T>::bytes() const {
-    size_t b = inv.bytes() + hinv.bytes() + cb.bytes() + cx.bytes() + cb64.bytes() + cx64.bytes() +
+    size_t b = inv.bytes() + hinv.bytes() + cb.bytes() + cx.bytes() +
                (sparse ? sparse->bytes() : 0);
     for (const auto& l : levels)
         b += l.A.bytes() + l.dinv.bytes() + l.pptr.bytes() + l.rptr.bytes() + l.pidx.bytes() +
@@ -2354,10 +2354,6 @@ void SolverImpl::tune_degree() {
 void SolverImpl::sparse_direct(const HostCsr& h, const std::vector<double>& xyz) {
     sparse_ = std::make_unique<SparseFactor>();
     sparse_->factor(h, xyz.data(), s_);
-    // The triangles of supernodes of 8 columns or more by products with their inverses: the
-    // direct solve of a 36,300-unknown P2 beam 3.7 against 5.9 ms, of a 32^3 heat cube 6.3
-    // against 9.6 ms.
-    sparse_->invert_blocks(8, s_);
 }
 
 void SolverImpl::dense_direct(const HostCsr& h) {
@@ -2559,16 +2555,9 @@ void SolverImpl::build_levels(const std::vector<const DevCsr*>& mats, std::vecto
         H->ncoarse = last.n;
         H->sparse = std::make_unique<SparseFactor>();
         H->sparse->factor(last, xyz.data(), s_);
-        // Inside the V-cycle the large supernodes' triangles are applied by products with their
-        // inverses (parallel) rather than by substitution column by column.
-        H->sparse->invert_blocks(8, s_);
         H->cb.alloc(last.n);
         H->cb.zero(s_);
         H->cx.alloc(last.n);
-        if (!std::is_same<T, double>::value) {
-            H->cb64.alloc(last.n);
-            H->cx64.alloc(last.n);
-        }
         FG_CUDA(cudaStreamSynchronize(s_));
         return;
     }
@@ -2776,14 +2765,7 @@ const T* SolverImpl::enqueue_vcycle(Hierarchy<T>& H, size_t l, const T* b, bool 
         // The sparse coarsest factor's 2 triangular solves in FP64 (the right side and the
         // solution converted in the mixed form).
         const int64_t n = H.ncoarse;
-        if constexpr (std::is_same<T, double>::value) {
-            H.sparse->solve(b, H.cx.p, s_);
-        } else {
-            k_convert<T, double><<<blocks_for(n, TH), TH, 0, s_>>>(n, b, H.cb64.p);
-            H.sparse->solve(H.cb64.p, H.cx64.p, s_);
-            k_convert<double, T><<<blocks_for(n, TH), TH, 0, s_>>>(n, H.cx64.p, H.cx.p);
-            launches_ += 2;
-        }
+        H.sparse->solve(b, H.cx.p, pdl_, s_);
         FG_CHECK_LAUNCH();
         mark("coarsest sparse solve n=" + std::to_string(n));
         launches_ += H.sparse->solve_launches();
@@ -3089,7 +3071,7 @@ void SolverImpl::solve_host_zero(const double* h_b, double* h_x, const volatile 
 void SolverImpl::precondition(const double* d_r, double* d_z) {
     FG_CUDA(cudaMemsetAsync(&sc_.p->done, 0, sizeof(int), s_));
     if (direct_ && sparse_) {
-        sparse_->solve(d_r, d_z, s_);
+        sparse_->solve(d_r, d_z, pdl_, s_);
     } else if (direct_) {
         k_gemv<double><<<blocks_for(n_ * 32, TH), TH, 0, s_>>>(n_, n_, dense_inv_.p, d_r, d_z,
                                                                done_zero_.p);
@@ -3121,7 +3103,7 @@ void SolverImpl::solve(const double* d_b, double* d_x, const volatile int* cance
         // residual.
         auto apply = [&](const double* rhs, double* sol) {
             if (sparse_) {
-                sparse_->solve(rhs, sol, s_);
+                sparse_->solve(rhs, sol, pdl_, s_);
             } else {
                 k_gemv<double><<<blocks_for(n * 32, TH), TH, 0, s_>>>(
                     n, n, dense_inv_.p, rhs, sol, done_zero_.p);

@@ -200,7 +200,6 @@ struct Hierarchy {
     // layers of an extruded footprint): its sparse multifrontal factor, as the reference's
     // coarsest solve (multigrid.rs:130-131), applied in FP64.
     std::unique_ptr<SparseFactor> sparse;
-    DevBuf<double> cb64, cx64;
     // The levels from `tail_from` down, and the coarsest solve, run as 1 cooperative kernel
     // (-1: none) of `tail_grid` blocks.
     int tail_from = -1, tail_grid = 0;

@@ -130,398 +130,267 @@ __global__ void __launch_bounds__(TH)
     for (int t = threadIdx.x; t < m * m; t += blockDim.x) F[t] = S[t];
 }
 
-__global__ void k_permute_in(int64_t n, const int64_t* __restrict__ perm,
-                             const double* __restrict__ b, double* __restrict__ y) {
-    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n;
-         j += (int64_t)gridDim.x * blockDim.x)
-        y[j] = b[perm[j]];
+// ---------------------------------------------------------------- the triangular solves
+// Each supernode keeps G = [W; L21 W] (m x k, column-major, leading dimension ld), W = L11^-1:
+// with z the supernode's right side (its part of b and its children's updates), the forward
+// solve is y1 = W z and z2 -= (L21 W) z, the backward one x1 = G^T [y1; -x2] with x2 the solved
+// rows below, stored with the sign in G's lower part (G = [W; -L21 W]). Both are 1 product, so
+// every row chunk (or column chunk) of a supernode is its own task with no order between them,
+// and a level of the tree is 1 launch over all the level's tasks. A block of 16 warps takes 1
+// task with 16 warps, 4 with 4, or 16 with 1, by the supernode's size.
+//
+// What bounds it: the factor is read once per direction (107 MB for the 36,300-unknown P2 beam:
+// 17 us at the copy bandwidth), but a launch per level and direction leaves each level with a
+// few microseconds of dependent latency. So each task loads its first entries of G and its
+// static indices before it waits for the level before (programmatic dependent launch); after the
+// wait only 1 round of loads (the right side) comes before the sums. The children's updates are
+// left in slots grouped by the parent's row, so that the parent reads them as 1 contiguous run.
+// Measured on B200: the 50 x 5 x 5 P2 beam's direct solve (2 applications of the factor, 36,300
+// unknowns) 3.70 -> 0.80 ms with 22 levels, 0.56 ms with the 11 levels of relaxed supernodes
+// (symbolic.cpp); the 29,910-unknown coarsest level of a prism mesh 1,633 -> 393 -> 199 us, its
+// kernels timed one by one. Before, 1 block took a whole supernode and the large ones near the
+// root left the other SMs idle. The error of 1 application against extended precision stayed:
+// 1e-12 to 6e-11 on P2 beams of 14,580 to 37,440 unknowns on either form.
+constexpr int SOLVE_WARPS = 16;
+constexpr int SOLVE_TH = 32 * SOLVE_WARPS;
+constexpr int ZCAP = 128;  // right side values staged per warp of a task
+constexpr int BATCH = 8;   // entries of G in flight per thread
+// Columns per warp of a backward task of 1 and of 4 warps (16 warps: 1).
+constexpr int COLS_1 = 4, COLS_4 = 2;
+
+__device__ __forceinline__ double slot_sum(double z, const double* slot, uint32_t e0,
+                                           uint32_t e1) {
+    for (uint32_t e = e0; e < e1; ++e) z += slot[e];
+    return z;
 }
 
-__global__ void k_permute_out(int64_t n, const int64_t* __restrict__ perm,
-                              const double* __restrict__ y, double* __restrict__ x) {
-    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n;
-         j += (int64_t)gridDim.x * blockDim.x)
-        x[perm[j]] = y[j];
-}
-
-// The product forms of a supernode's triangular solves, when the inverse W = L11^-1 of its
-// diagonal block is kept (k x k, column-major): z1 = W z1 and z2 -= L21 z1 in the forward
-// direction, x1 = W^T t in the backward one. The vector is staged in shared memory 1024 values
-// at a time; tmp is the supernode's own range of a scratch vector (its columns j0 .. j0 + k).
-constexpr int ZS = 1024;
-
-__device__ void forward_by_inverse(const double* __restrict__ W, const double* __restrict__ F,
-                                   int64_t m, int64_t k, double* __restrict__ z,
-                                   double* __restrict__ tmp) {
-    __shared__ double zs[ZS];
-    for (int64_t i = threadIdx.x; i < k; i += blockDim.x) tmp[i] = 0.0;
-    for (int64_t c0 = 0; c0 < k; c0 += ZS) {
-        const int cnt = (int)min((int64_t)ZS, k - c0);
+// A level of the forward solve: task = 32 rows of a supernode, a lane per row, the warps of the
+// task splitting its columns.
+template <class TB>
+__global__ void __launch_bounds__(SOLVE_TH)
+    k_sparse_forward(const SolveBlock* __restrict__ blocks, const SolveTask* __restrict__ tasks,
+                     const double* __restrict__ G, const uint32_t* __restrict__ slot_ptr,
+                     const uint32_t* __restrict__ dst, const int64_t* __restrict__ perm,
+                     const TB* b, double* slot, double* yf) {
+    __shared__ double zs[SOLVE_WARPS * ZCAP];
+    __shared__ double red[SOLVE_TH];
+    const SolveBlock B = blocks[blockIdx.x];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nw = B.warps, group = warp / nw, wg = warp % nw;
+    SolveTask t{};
+    if (group < B.count) t = tasks[B.task + group];
+    const int row = t.at + lane;
+    const bool mine = row < t.m;
+    const int kc = min(t.k, t.at + 32);  // W is lower triangular
+    const double* col = G + t.g + row;
+    double g[BATCH];
+#pragma unroll
+    for (int u = 0; u < BATCH; ++u) {
+        const int j = wg + u * nw;
+        g[u] = mine && j < kc ? col[(int64_t)j * t.ld] : 0.0;
+    }
+    const int tid = wg * 32 + lane, gt = nw * 32, cap = ZCAP * nw;
+    double* z = zs + group * cap;
+    uint32_t e0 = 0, e1 = 0, s0 = 0, s1 = 0, d = 0;
+    int64_t pi = 0;
+    if (tid < kc) {
+        e0 = slot_ptr[t.z + tid];
+        e1 = slot_ptr[t.z + tid + 1];
+        pi = perm[t.j0 + tid];
+    }
+    if (wg == 0 && mine && row >= t.k) {
+        s0 = slot_ptr[t.z + row];
+        s1 = slot_ptr[t.z + row + 1];
+        d = dst[t.z + row];
+    }
+    pdl_wait();
+    double acc = 0.0;
+    // Tasks of fewer than 16 warps have at most `cap` columns: 1 turn for all of the block's.
+    const int turns = nw == SOLVE_WARPS ? max(1, (kc + cap - 1) / cap) : 1;
+    for (int turn = 0; turn < turns; ++turn) {
+        const int c0 = turn * cap, c1 = min(kc, c0 + cap);
+        for (int i = c0 + tid; i < c1; i += gt) {
+            if (i != tid) {
+                e0 = slot_ptr[t.z + i];
+                e1 = slot_ptr[t.z + i + 1];
+                pi = perm[t.j0 + i];
+            }
+            z[i - c0] = slot_sum((double)b[pi], slot, e0, e1);
+        }
         __syncthreads();
-        for (int t = threadIdx.x; t < cnt; t += blockDim.x) zs[t] = z[c0 + t];
+        int j = c0 + wg;
+        if (turn == 0) {
+#pragma unroll
+            for (int u = 0; u < BATCH; ++u) {
+                if (j < c1) acc += g[u] * z[j];
+                j += nw;
+            }
+        }
+        for (; j < c1; j += BATCH * nw) {
+#pragma unroll
+            for (int u = 0; u < BATCH; ++u) {
+                const int c = j + u * nw;
+                g[u] = mine && c < c1 ? col[(int64_t)c * t.ld] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < BATCH; ++u) {
+                const int c = j + u * nw;
+                if (c < c1) acc += g[u] * z[c - c0];
+            }
+        }
         __syncthreads();
-        for (int64_t i = c0 + threadIdx.x; i < k; i += blockDim.x) {
-            const int hi = (int)min((int64_t)cnt, i - c0 + 1);  // W lower: j <= i
-            double acc = 0.0;
-            for (int j = 0; j < hi; ++j) acc += W[i + (c0 + j) * k] * zs[j];
-            tmp[i] += acc;
+    }
+    if (nw > 1) {
+        red[threadIdx.x] = acc;
+        __syncthreads();
+        if (wg == 0) {
+            acc = 0.0;
+            for (int w = 0; w < nw; ++w) acc += red[(warp + w) * 32 + lane];
         }
     }
-    __syncthreads();
-    for (int64_t i = threadIdx.x; i < k; i += blockDim.x) z[i] = tmp[i];
-    // z2 -= L21 z1, z1 staged again.
-    for (int64_t c0 = 0; c0 < k; c0 += ZS) {
-        const int cnt = (int)min((int64_t)ZS, k - c0);
-        __syncthreads();
-        for (int t = threadIdx.x; t < cnt; t += blockDim.x) zs[t] = z[c0 + t];
-        __syncthreads();
-        for (int64_t r = k + threadIdx.x; r < m; r += blockDim.x) {
-            double acc = 0.0;
-            for (int j = 0; j < cnt; ++j) acc += F[r + (c0 + j) * m] * zs[j];
-            z[r] -= acc;
-        }
+    if (wg == 0 && mine) {
+        if (row < t.k)
+            yf[t.j0 + row] = acc;
+        else
+            slot[d] = slot_sum(0.0, slot, s0, s1) + acc;
     }
-    __syncthreads();
 }
 
-__device__ void backward_by_inverse(const double* __restrict__ W, int64_t k,
-                                    double* __restrict__ z, double* __restrict__ tmp) {
-    __shared__ double ts[ZS];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int64_t j = threadIdx.x; j < k; j += blockDim.x) tmp[j] = 0.0;
-    for (int64_t c0 = 0; c0 < k; c0 += ZS) {
-        const int cnt = (int)min((int64_t)ZS, k - c0);
-        __syncthreads();
-        for (int t = threadIdx.x; t < cnt; t += blockDim.x) ts[t] = z[c0 + t];
-        __syncthreads();
-        // x1[j] += sum over rows i of the chunk with i >= j of W[i][j] t[i] (column j of W is
-        // contiguous): a warp per column.
-        for (int64_t j = warp; j < k && j < c0 + cnt; j += nw) {
-            const int lo = (int)max((int64_t)0, j - c0);
-            const double* col = W + c0 + j * k;
-            double acc = 0.0;
-            for (int t = lo + lane; t < cnt; t += 32) acc += col[t] * ts[t];
-            for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-            if (lane == 0) tmp[j] += acc;
+// A task of the backward solve: up to C columns per warp of a supernode, the lanes along the
+// rows, U rows of each column in flight per lane.
+template <int C, int U, class TX>
+__device__ __forceinline__ void backward_task(const SolveTask& t, int nw, int wg, int lane,
+                                              double* v, const double* __restrict__ G,
+                                              const uint32_t* __restrict__ rows,
+                                              const int64_t* __restrict__ perm,
+                                              const double* yf, double* xs, TX* x) {
+    // Column c of the task is column at + c of G; W is lower triangular, so its rows above at
+    // are 0.
+    const int i0 = t.at & ~3;
+    const double* col[C];
+    bool on[C];
+    double g[U][C], acc[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        const int j = wg + c * nw;
+        on[c] = j < t.cols;
+        col[c] = G + t.g + (int64_t)(t.at + j) * t.ld;
+        acc[c] = 0.0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int i = i0 + 32 * u + lane;
+            g[u][c] = on[c] && i < t.m ? col[c][i] : 0.0;
         }
     }
-    __syncthreads();
-    for (int64_t j = threadIdx.x; j < k; j += blockDim.x) z[j] = tmp[j];
-    __syncthreads();
+    const int tid = wg * 32 + lane, gt = nw * 32, cap = ZCAP * nw;
+    uint32_t r = 0;
+    if (i0 + tid < t.m && i0 + tid >= t.k) r = rows[t.z + i0 + tid];
+    pdl_wait();
+    // Tasks of fewer than 16 warps have at most `cap` rows: 1 turn for all of the block's.
+    const int turns = nw == SOLVE_WARPS ? max(1, (t.m - i0 + cap - 1) / cap) : 1;
+    for (int turn = 0; turn < turns; ++turn) {
+        const int c0 = i0 + turn * cap, c1 = min(t.m, c0 + cap);
+        for (int i = c0 + tid; i < c1; i += gt) {
+            if (i >= t.k && i != i0 + tid) r = rows[t.z + i];
+            v[i - c0] = i < t.k ? yf[t.j0 + i] : xs[r];
+        }
+        __syncthreads();
+        for (int i = c0; i < c1; i += 32 * U) {
+            if (i != i0) {
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+#pragma unroll
+                    for (int c = 0; c < C; ++c)
+                        g[u][c] = on[c] && i + 32 * u + lane < c1 ? col[c][i + 32 * u + lane] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int q = i + 32 * u + lane;
+                const double vi = q < c1 ? v[q - c0] : 0.0;
+#pragma unroll
+                for (int c = 0; c < C; ++c) acc[c] += g[u][c] * vi;
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        double a = acc[c];
+#pragma unroll
+        for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        if (lane == 0 && on[c]) {
+            const int64_t j = t.j0 + t.at + wg + c * nw;
+            xs[j] = a;
+            x[perm[j]] = (TX)a;
+        }
+    }
 }
 
-// Forward solve of supernode s (1 block): z = its part of y and its children's updates (added
-// child by child in increasing order), then L11 z1 = z1 and z2 -= L21 z1 by blocks of 32 columns;
-// z1 goes to y, z2 is the update for the parent.
-__global__ void __launch_bounds__(TH)
-    k_forward(const int64_t* __restrict__ list, Fronts fr, const int64_t* __restrict__ zoff,
-              const int64_t* __restrict__ child_ptr, const int64_t* __restrict__ child,
-              const uint32_t* __restrict__ relind, const int64_t* __restrict__ relind_off,
-              double* __restrict__ work, double* __restrict__ y,
-              const int64_t* __restrict__ winv_off, const double* __restrict__ winv,
-              double* __restrict__ tmp) {
+// A level of the backward solve.
+template <class TX>
+__global__ void __launch_bounds__(SOLVE_TH)
+    k_sparse_backward(const SolveBlock* __restrict__ blocks, const SolveTask* __restrict__ tasks,
+                      const double* __restrict__ G, const uint32_t* __restrict__ rows,
+                      const int64_t* __restrict__ perm, const double* yf, double* xs, TX* x) {
+    __shared__ double vs[SOLVE_WARPS * ZCAP];
+    const SolveBlock B = blocks[blockIdx.x];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nw = B.warps, group = warp / nw, wg = warp % nw;
+    SolveTask t{};
+    if (group < B.count) t = tasks[B.task + group];
+    double* v = vs + group * ZCAP * nw;
+    if (nw == 1)
+        backward_task<COLS_1, 2>(t, nw, wg, lane, v, G, rows, perm, yf, xs, x);
+    else if (nw == 4)
+        backward_task<COLS_4, 4>(t, nw, wg, lane, v, G, rows, perm, yf, xs, x);
+    else
+        backward_task<1, 8>(t, nw, wg, lane, v, G, rows, perm, yf, xs, x);
+}
+
+// ---------------------------------------------------------------- the form of the solves
+
+// G of a supernode of at most 32 columns: 1 block. W by forward substitution, a lane of the
+// first warp per column; then a thread per row of -L21 W, its row of L21 in registers.
+constexpr int INV_SMALL = 32;
+__global__ void __launch_bounds__(128)
+    k_small_inverse(const int64_t* __restrict__ list, Fronts fr, const int64_t* __restrict__ goff,
+                    const int64_t* __restrict__ gld, double* __restrict__ G) {
+    __shared__ double L[INV_SMALL][INV_SMALL + 1], W[INV_SMALL][INV_SMALL + 1];
     const int64_t s = list[blockIdx.x];
-    const int64_t j0 = fr.first[s];
-    const int64_t m = fr.rows_ptr[s + 1] - fr.rows_ptr[s], k = fr.first[s + 1] - j0;
+    const int64_t m = fr.rows_ptr[s + 1] - fr.rows_ptr[s], ld = gld[s];
+    const int k = (int)(fr.first[s + 1] - fr.first[s]);
     const double* F = fr.f + fr.foff[s];
-    double* z = work + zoff[s];
-    for (int64_t t = threadIdx.x; t < m; t += blockDim.x) z[t] = t < k ? y[j0 + t] : 0.0;
+    double* g = G + goff[s];
+    for (int e = threadIdx.x; e < INV_SMALL * INV_SMALL; e += blockDim.x) {
+        const int i = e % INV_SMALL, j = e / INV_SMALL;
+        L[i][j] = i < k && j <= i ? F[i + j * m] : 0.0;
+        W[i][j] = 0.0;
+    }
     __syncthreads();
-    for (int64_t ci = child_ptr[s]; ci < child_ptr[s + 1]; ++ci) {
-        const int64_t c = child[ci];
-        const int64_t kc = fr.first[c + 1] - fr.first[c];
-        const int64_t mu = fr.rows_ptr[c + 1] - fr.rows_ptr[c] - kc;
-        const double* zc = work + zoff[c] + kc;
-        const uint32_t* rel = relind + relind_off[c];
-        for (int64_t t = threadIdx.x; t < mu; t += blockDim.x) z[rel[t]] += zc[t];
-        __syncthreads();
-    }
-    if (winv_off && winv_off[s] >= 0) {
-        forward_by_inverse(winv + winv_off[s], F, m, k, z, tmp + j0);
-        for (int64_t t = threadIdx.x; t < k; t += blockDim.x) y[j0 + t] = z[t];
-        return;
-    }
-    // The columns in blocks of 32: warp 0 solves the block's triangle with shuffles (lane i
-    // holds row jb + i), then every thread takes rows below the block and subtracts the block's
-    // 32 columns times the solved values: 2 barriers per 32 columns instead of 2 per column.
-    __shared__ double zb[32];
-    for (int64_t jb = 0; jb < k; jb += 32) {
-        const int kb = (int)min((int64_t)32, k - jb);
-        if (threadIdx.x < 32) {
-            // Lane l holds row jb + l of the block's triangle in registers (all loads issued
-            // before the serial steps, which then only shuffle).
-            const int l = threadIdx.x;
-            double row[32];
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-                row[j] = (j < kb && l < kb && j <= l) ? F[(jb + l) + (jb + j) * m] : 0.0;
-            double x = l < kb ? z[jb + l] : 0.0;
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                if (j < kb) {
-                    if (l == j) x = x / row[j];
-                    const double xj = __shfl_sync(0xffffffffu, x, j);
-                    if (l > j) x -= row[j] * xj;
-                }
-            }
-            if (l < kb) {
-                z[jb + l] = x;
-                zb[l] = x;
-            }
-        }
-        __syncthreads();
-        for (int64_t r = jb + kb + threadIdx.x; r < m; r += blockDim.x) {
-            double acc = 0.0;
-            for (int j = 0; j < kb; ++j) acc += F[r + (jb + j) * m] * zb[j];
-            z[r] -= acc;
-        }
-        __syncthreads();
-    }
-    for (int64_t t = threadIdx.x; t < k; t += blockDim.x) y[j0 + t] = z[t];
-}
-
-// Backward solve of supernode s (1 block), its ancestors done: t_j = y_j - sum over the rows
-// below of L[r][j] x_r (a warp per column), then L11^T x1 = t.
-__global__ void __launch_bounds__(TH)
-    k_backward(const int64_t* __restrict__ list, Fronts fr, const int64_t* __restrict__ zoff,
-               double* __restrict__ work, double* __restrict__ y,
-               const int64_t* __restrict__ winv_off, const double* __restrict__ winv,
-               double* __restrict__ tmp) {
-    const int64_t s = list[blockIdx.x];
-    const int64_t j0 = fr.first[s];
-    const int64_t r0 = fr.rows_ptr[s];
-    const int64_t m = fr.rows_ptr[s + 1] - r0, k = fr.first[s + 1] - j0;
-    const uint32_t* R = fr.rows + r0;
-    const double* F = fr.f + fr.foff[s];
-    double* z = work + zoff[s];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    // The solved values of the rows below (y at R[r], r >= k) gathered into shared memory a
-    // chunk at a time, so that each warp's column sums read the front coalesced and x from
-    // shared memory, with no dependent global loads.
-    constexpr int XG = 1024;
-    __shared__ double xg[XG];
-    for (int64_t t = threadIdx.x; t < k; t += blockDim.x) z[t] = y[j0 + t];
-    for (int64_t r0 = k; r0 < m; r0 += XG) {
-        const int cnt = (int)min((int64_t)XG, m - r0);
-        __syncthreads();
-        for (int t = threadIdx.x; t < cnt; t += blockDim.x) xg[t] = y[R[r0 + t]];
-        __syncthreads();
-        for (int64_t j = warp; j < k; j += nw) {
-            const double* col = F + r0 + j * m;
-            double acc = 0.0;
-            for (int t = lane; t < cnt; t += 32) acc += col[t] * xg[t];
-            for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-            if (lane == 0) z[j] -= acc;
+    if (threadIdx.x < k) {
+        const int c = threadIdx.x;
+        for (int i = c; i < k; ++i) {
+            double v = i == c ? 1.0 : 0.0;
+            for (int j = c; j < i; ++j) v -= L[i][j] * W[j][c];
+            W[i][c] = v / L[i][i];
         }
     }
     __syncthreads();
-    if (winv_off && winv_off[s] >= 0) {
-        backward_by_inverse(winv + winv_off[s], k, z, tmp + j0);
-        for (int64_t t = threadIdx.x; t < k; t += blockDim.x) y[j0 + t] = z[t];
-        return;
-    }
-    // L11^T x1 = t in blocks of 32 from the last: warp 0 solves the block's triangle with
-    // shuffles, then every row above the block subtracts the block's solved values times its
-    // row of L (the 32 entries contiguous in the column-major front).
-    __shared__ double zb[32];
-    for (int64_t je = k; je > 0; je -= 32) {
-        const int64_t jb = je >= 32 ? je - 32 : 0;
-        const int kb = (int)(je - jb);
-        if (threadIdx.x < 32) {
-            // Lane l holds column jb + l of the block's triangle (contiguous in the front).
-            const int l = threadIdx.x;
-            double col[32];
+    for (int e = threadIdx.x; e < k * k; e += blockDim.x) g[e % k + (e / k) * ld] = W[e % k][e / k];
+    for (int64_t r = k + threadIdx.x; r < m; r += blockDim.x) {
+        double l[INV_SMALL];
 #pragma unroll
-            for (int j = 0; j < 32; ++j)
-                col[j] = (j < kb && l < kb && j >= l) ? F[(jb + j) + (jb + l) * m] : 0.0;
-            double x = l < kb ? z[jb + l] : 0.0;
+        for (int j = 0; j < INV_SMALL; ++j) l[j] = j < k ? F[r + j * m] : 0.0;
+        for (int c = 0; c < k; ++c) {
+            double v = 0.0;
 #pragma unroll
-            for (int j = 31; j >= 0; --j) {
-                if (j < kb) {
-                    if (l == j) x = x / col[j];
-                    const double xj = __shfl_sync(0xffffffffu, x, j);
-                    if (l < j) x -= col[j] * xj;
-                }
-            }
-            if (l < kb) {
-                z[jb + l] = x;
-                zb[l] = x;
-            }
+            for (int j = 0; j < INV_SMALL; ++j) v -= l[j] * W[j][c];
+            g[r + c * ld] = v;
         }
-        __syncthreads();
-        for (int64_t i = threadIdx.x; i < jb; i += blockDim.x) {
-            double acc = 0.0;
-            for (int j = 0; j < kb; ++j) acc += F[(jb + j) + i * m] * zb[j];
-            z[i] -= acc;
-        }
-        __syncthreads();
     }
-    for (int64_t t = threadIdx.x; t < k; t += blockDim.x) y[j0 + t] = z[t];
+    for (int64_t r = m + threadIdx.x; r < ld; r += blockDim.x)
+        for (int c = 0; c < k; ++c) g[r + c * ld] = 0.0;
 }
-
-}  // namespace
-
-void SparseFactor::factor(const HostCsr& a, const double* xyz, cudaStream_t s) {
-    n_ = a.n;
-    // The reference's fill-reducing order (order.rs) and the analysis in it.
-    Supernodal S = analyse_factor(a, nested_dissection(a, xyz));
-    ns_ = S.ns;
-    entries_ = S.entries;
-    flops_ = S.flops;
-    host_first_ = S.first;
-    m_.resize(ns_);
-    k_.resize(ns_);
-    std::vector<int64_t> foff(ns_), zoff(ns_);
-    size_t fv = 0, zv = 0;
-    for (int64_t t = 0; t < ns_; ++t) {
-        m_[t] = S.rows_ptr[t + 1] - S.rows_ptr[t];
-        k_[t] = S.first[t + 1] - S.first[t];
-        foff[t] = (int64_t)fv;
-        zoff[t] = (int64_t)zv;
-        fv += (size_t)(m_[t] * m_[t]);
-        zv += (size_t)m_[t];
-    }
-    front_values_ = fv;
-    if (fv > ((size_t)96 << 30) / 8)
-        throw Failure(FEMGPU_ERR_TOO_LARGE,
-                      "the frontal matrices of the sparse factor need more than 96 GiB");
-    // Children (increasing), relative indices of each child's update rows in its parent.
-    std::vector<int64_t> cptr(ns_ + 1, 0), clist;
-    for (int64_t t = 0; t < ns_; ++t)
-        if (S.parent[t] >= 0) cptr[S.parent[t] + 1] += 1;
-    for (int64_t t = 0; t < ns_; ++t) cptr[t + 1] += cptr[t];
-    clist.resize(cptr[ns_]);
-    std::vector<int64_t> fill(cptr.begin(), cptr.end() - 1);
-    std::vector<int> rank(ns_, 0);
-    for (int64_t t = 0; t < ns_; ++t)
-        if (S.parent[t] >= 0) {
-            rank[t] = (int)(fill[S.parent[t]] - cptr[S.parent[t]]);
-            clist[fill[S.parent[t]]++] = t;
-        }
-    std::vector<int64_t> roff(ns_, 0);
-    std::vector<uint32_t> rel;
-    for (int64_t c = 0; c < ns_; ++c) {
-        roff[c] = (int64_t)rel.size();
-        const int64_t p = S.parent[c];
-        if (p < 0) continue;
-        const uint32_t* Rp = S.rows.data() + S.rows_ptr[p];
-        for (int64_t t = S.rows_ptr[c] + k_[c]; t < S.rows_ptr[c + 1]; ++t)
-            rel.push_back((uint32_t)(std::lower_bound(Rp, Rp + m_[p], S.rows[t]) - Rp));
-    }
-    // The level schedule.
-    height_ = 0;
-    for (int h : S.height) height_ = std::max<int64_t>(height_, h);
-    small_.assign(height_ + 1, {});
-    large_.assign(height_ + 1, {});
-    std::vector<std::vector<int64_t>> all(height_ + 1);
-    for (int64_t t = 0; t < ns_; ++t) {
-        (m_[t] <= SMALL_ROWS ? small_ : large_)[S.height[t]].push_back(t);
-        all[S.height[t]].push_back(t);
-    }
-    std::vector<int64_t> sl, ll;
-    small_at_.assign(1, 0);
-    level_at_.assign(1, 0);
-    for (int64_t h = 0; h <= height_; ++h) {
-        sl.insert(sl.end(), small_[h].begin(), small_[h].end());
-        small_at_.push_back((int64_t)sl.size());
-        ll.insert(ll.end(), all[h].begin(), all[h].end());
-        level_at_.push_back((int64_t)ll.size());
-    }
-    // Extend-add chunks per (height of the parent, rank of the child).
-    std::vector<int2> ch;
-    chunks_.clear();
-    for (int64_t h = 1; h <= height_; ++h) {
-        int maxrank = -1;
-        for (int64_t p : all[h]) maxrank = std::max<int>(maxrank, (int)(cptr[p + 1] - cptr[p]) - 1);
-        for (int r = 0; r <= maxrank; ++r) {
-            Chunks c{(int)h, r, (int64_t)ch.size(), 0};
-            for (int64_t p : all[h]) {
-                if (cptr[p + 1] - cptr[p] <= r) continue;
-                const int64_t cc = clist[cptr[p] + r];
-                const int64_t mu = m_[cc] - k_[cc];
-                const int64_t parts = (mu * mu + CHUNK - 1) / CHUNK;
-                for (int64_t q = 0; q < parts; ++q) ch.push_back(int2{(int)cc, (int)q});
-            }
-            c.count = (int64_t)ch.size() - c.at;
-            if (c.count) chunks_.push_back(c);
-        }
-    }
-    if (ns_ >= INT_MAX) throw Failure(FEMGPU_ERR_TOO_LARGE, "too many supernodes");
-    // Device arrays.
-    std::vector<int32_t> col2sn(n_);
-    for (int64_t t = 0; t < ns_; ++t)
-        for (int64_t j = S.first[t]; j < S.first[t + 1]; ++j) col2sn[j] = (int32_t)t;
-    perm_.upload(S.perm.data(), n_, s);
-    DevBuf<int64_t> iperm;
-    iperm.upload(S.iperm.data(), n_, s);
-    first_.upload(S.first.data(), ns_ + 1, s);
-    rows_ptr_.upload(S.rows_ptr.data(), ns_ + 1, s);
-    rows_.upload(S.rows.data(), S.rows.size(), s);
-    foff_.upload(foff.data(), ns_, s);
-    host_foff_ = foff;
-    zoff_.upload(zoff.data(), ns_, s);
-    child_ptr_.upload(cptr.data(), ns_ + 1, s);
-    child_.upload(clist.data(), std::max<size_t>(1, clist.size()), s);
-    relind_.upload(rel.data(), std::max<size_t>(1, rel.size()), s);
-    relind_off_.upload(roff.data(), ns_, s);
-    small_list_.upload(sl.data(), std::max<size_t>(1, sl.size()), s);
-    level_list_.upload(ll.data(), std::max<size_t>(1, ll.size()), s);
-    chunk_.upload(ch.data(), std::max<size_t>(1, ch.size()), s);
-    DevBuf<int64_t> parent;
-    parent.upload(S.parent.data(), ns_, s);
-    DevBuf<int32_t> dcol2sn;
-    dcol2sn.upload(col2sn.data(), n_, s);
-    fronts_.alloc(fv);
-    FG_CUDA(cudaMemsetAsync(fronts_.p, 0, fv * sizeof(double), s));
-    work_.alloc(std::max<size_t>(1, zv));
-    y_.alloc(n_);
-    DevBuf<int64_t> aptr;
-    DevBuf<uint32_t> aidx;
-    DevBuf<double> aval, diag0(n_);
-    aptr.upload(a.ptr.data(), n_ + 1, s);
-    aidx.upload(a.idx.data(), a.nnz(), s);
-    aval.upload(a.val.data(), a.nnz(), s);
-    DevBuf<unsigned long long> status(1);
-    FG_CUDA(cudaMemsetAsync(status.p, 0xff, sizeof(unsigned long long), s));
-    const Fronts fr{first_.p, rows_ptr_.p, rows_.p, foff_.p, fronts_.p};
-    k_assemble_fronts<<<blocks_for(n_, TH), TH, 0, s>>>(n_, perm_.p, iperm.p, aptr.p, aidx.p,
-                                                       aval.p, dcol2sn.p, fr, diag0.p);
-    FG_CHECK_LAUNCH();
-    const size_t smem = (size_t)SMALL_ROWS * SMALL_ROWS * sizeof(double);
-    FG_CUDA(cudaFuncSetAttribute(k_front_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
-    size_t ci = 0;
-    for (int64_t h = 0; h <= height_; ++h) {
-        for (; ci < chunks_.size() && chunks_[ci].height == h; ++ci)
-            k_extend_add<<<(unsigned)chunks_[ci].count, TH, 0, s>>>(
-                chunk_.p + chunks_[ci].at, fr, parent.p, relind_.p, relind_off_.p);
-        const int64_t ns_small = small_at_[h + 1] - small_at_[h];
-        if (ns_small > 0) {
-            int mmax = 0;
-            for (int64_t t : small_[h]) mmax = std::max<int>(mmax, (int)m_[t]);
-            k_front_small<<<(unsigned)ns_small, TH, (size_t)mmax * mmax * sizeof(double), s>>>(
-                small_list_.p + small_at_[h], fr, diag0.p, status.p);
-        }
-        for (int64_t t : large_[h])
-            dense_partial_cholesky(fronts_.p + foff[t], m_[t], k_[t], diag0.p + S.first[t],
-                                   S.first[t], status.p, s);
-        FG_CHECK_LAUNCH();
-    }
-    unsigned long long bad = fetch(status.p, s);
-    if (bad != ~0ull) {
-        const int64_t j = (int64_t)bad;
-        const double d = fetch(diag0.p + j, s);
-        char buf[320];
-        std::snprintf(buf, sizeof buf,
-                      "the matrix is not positive definite: the pivot of column %lld is 0 or less "
-                      "to the precision of the arithmetic (its diagonal is %s)",
-                      (long long)S.perm[j], rust_exp_shortest(d).c_str());
-        throw Failure(FEMGPU_ERR_NOT_SPD, buf);
-    }
-    FG_CUDA(cudaStreamSynchronize(s));
-}
-
-namespace {
 
 // The lower triangle of the k x k diagonal block of front F (leading dimension m) into L (leading
 // dimension k), zeros above: 1 member of the copy per blockIdx.y.
@@ -540,90 +409,381 @@ __global__ void k_copy_blocks(const BlockCopy* __restrict__ c) {
     }
 }
 
+// G of the larger supernodes from their W, in 64 x 64 tiles: W itself, or -L21 W summed over the
+// columns in order.
+struct GTile {
+    const double *F, *W;
+    double* g;
+    int64_t m, k, ld;
+    int r0, c0;
+};
+
+__global__ void __launch_bounds__(TH) k_large_panel(const GTile* __restrict__ tiles) {
+    constexpr int KT = 16;
+    __shared__ double A[KT][64], Bs[KT][64 + 1];
+    const GTile t = tiles[blockIdx.x];
+    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+    double acc[4][4] = {};
+    // W is lower triangular: its column c starts at row c.
+    for (int64_t k0 = t.c0; k0 < t.k; k0 += KT) {
+        for (int e = threadIdx.x; e < KT * 64; e += TH) {
+            const int r = e % 64, q = e / 64;
+            const int64_t i = t.r0 + r;
+            // L21, or the identity where the tile's rows are W's own.
+            A[q][r] = k0 + q < t.k && i < t.m
+                          ? (i < t.k ? (i == k0 + q ? -1.0 : 0.0) : t.F[i + (k0 + q) * t.m])
+                          : 0.0;
+        }
+        for (int e = threadIdx.x; e < KT * 64; e += TH) {
+            const int q = e % KT, c = e / KT;
+            Bs[q][c] = k0 + q < t.k && t.c0 + c < t.k ? t.W[k0 + q + (t.c0 + c) * t.k] : 0.0;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < KT; ++q)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] -= A[q][tx + 16 * i] * Bs[q][ty + 16 * j];
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int64_t r = t.r0 + tx + 16 * i, c = t.c0 + ty + 16 * j;
+            if (r < t.ld && c < t.k) t.g[r + c * t.ld] = acc[i][j];
+        }
+}
+
 }  // namespace
 
-void SparseFactor::invert_blocks(int64_t min_cols, cudaStream_t s) {
-    std::vector<int64_t> off(ns_, -1);
-    std::vector<int64_t> members;
-    int64_t total = 0, kmax = 0;
-    for (int64_t t = 0; t < ns_; ++t)
-        if (k_[t] >= min_cols) {
-            off[t] = total;
-            total += k_[t] * k_[t];
-            members.push_back(t);
-            kmax = std::max(kmax, k_[t]);
-        }
-    if (members.empty()) return;
-    if (members.size() > 65535) throw Failure(FEMGPU_ERR_TOO_LARGE, "too many large supernodes");
-    winv_.alloc(total);
-    tmp_.alloc(std::max<int64_t>(n_, 1));
-    DevBuf<double> lc(total);
-    std::vector<BlockCopy> bc;
-    std::vector<int64_t> ns;
-    std::vector<double*> ls, ws;
-    for (int64_t t : members) {
-        bc.push_back({fronts_.p + host_foff_[t], lc.p + off[t], m_[t], k_[t]});
-        ns.push_back(k_[t]);
-        ls.push_back(lc.p + off[t]);
-        ws.push_back(winv_.p + off[t]);
+void SparseFactor::factor(const HostCsr& a, const double* xyz, cudaStream_t s) {
+    n_ = a.n;
+    // The reference's fill-reducing order (order.rs) and the analysis in it.
+    Supernodal S = analyse_factor(a, nested_dissection(a, xyz));
+    ns_ = S.ns;
+    entries_ = S.entries;
+    flops_ = S.flops;
+    m_.resize(ns_);
+    k_.resize(ns_);
+    std::vector<int64_t> foff(ns_);
+    size_t fv = 0;
+    for (int64_t t = 0; t < ns_; ++t) {
+        m_[t] = S.rows_ptr[t + 1] - S.rows_ptr[t];
+        k_[t] = S.first[t + 1] - S.first[t];
+        foff[t] = (int64_t)fv;
+        fv += (size_t)(m_[t] * m_[t]);
     }
-    DevBuf<BlockCopy> dbc;
-    dbc.upload(bc.data(), bc.size(), s);
-    k_copy_blocks<<<dim3((unsigned)blocks_for(kmax * kmax, TH, 256), (unsigned)bc.size()), TH, 0,
-                    s>>>(dbc.p);
+    front_values_ = fv;
+    if (fv > ((size_t)96 << 30) / 8)
+        throw Failure(FEMGPU_ERR_TOO_LARGE,
+                      "the frontal matrices of the sparse factor need more than 96 GiB");
+    // Children (increasing), relative indices of each child's update rows in its parent.
+    std::vector<int64_t> cptr(ns_ + 1, 0), clist;
+    for (int64_t t = 0; t < ns_; ++t)
+        if (S.parent[t] >= 0) cptr[S.parent[t] + 1] += 1;
+    for (int64_t t = 0; t < ns_; ++t) cptr[t + 1] += cptr[t];
+    clist.resize(cptr[ns_]);
+    std::vector<int64_t> fill(cptr.begin(), cptr.end() - 1);
+    for (int64_t t = 0; t < ns_; ++t)
+        if (S.parent[t] >= 0) clist[fill[S.parent[t]]++] = t;
+    std::vector<int64_t> roff(ns_, 0);
+    std::vector<uint32_t> rel;
+    for (int64_t c = 0; c < ns_; ++c) {
+        roff[c] = (int64_t)rel.size();
+        const int64_t p = S.parent[c];
+        if (p < 0) continue;
+        const uint32_t* Rp = S.rows.data() + S.rows_ptr[p];
+        for (int64_t t = S.rows_ptr[c] + k_[c]; t < S.rows_ptr[c + 1]; ++t)
+            rel.push_back((uint32_t)(std::lower_bound(Rp, Rp + m_[p], S.rows[t]) - Rp));
+    }
+    // The level schedule.
+    height_ = 0;
+    for (int h : S.height) height_ = std::max<int64_t>(height_, h);
+    std::vector<std::vector<int64_t>> small(height_ + 1), large(height_ + 1);
+    levels_.assign(height_ + 1, {});
+    large_fronts_ = 0;
+    for (int64_t t = 0; t < ns_; ++t) {
+        (m_[t] <= SMALL_ROWS ? small : large)[S.height[t]].push_back(t);
+        large_fronts_ += m_[t] > SMALL_ROWS;
+        levels_[S.height[t]].push_back(t);
+    }
+    std::vector<int64_t> sl, small_at(1, 0);
+    for (int64_t h = 0; h <= height_; ++h) {
+        sl.insert(sl.end(), small[h].begin(), small[h].end());
+        small_at.push_back((int64_t)sl.size());
+    }
+    // The slots of the forward solve: the update that row r of a supernode gets from each child,
+    // a row's slots together and in the children's order.
+    host_zoff_.assign(S.rows_ptr.begin(), S.rows_ptr.end() - 1);
+    const size_t nrows = S.rows.size();
+    if (nrows >= (size_t)UINT32_MAX) throw Failure(FEMGPU_ERR_TOO_LARGE, "too many factor rows");
+    std::vector<uint32_t> slot_ptr(nrows + 1, 0), dst(nrows, 0);
+    for (int64_t c = 0; c < ns_; ++c)
+        if (S.parent[c] >= 0)
+            for (int64_t t = 0; t < m_[c] - k_[c]; ++t)
+                slot_ptr[S.rows_ptr[S.parent[c]] + rel[roff[c] + t] + 1] += 1;
+    for (size_t t = 0; t < nrows; ++t) slot_ptr[t + 1] += slot_ptr[t];
+    std::vector<uint32_t> next(slot_ptr.begin(), slot_ptr.end() - 1);
+    for (int64_t c = 0; c < ns_; ++c)
+        if (S.parent[c] >= 0)
+            for (int64_t t = 0; t < m_[c] - k_[c]; ++t)
+                dst[S.rows_ptr[c] + k_[c] + t] =
+                    next[S.rows_ptr[S.parent[c]] + rel[roff[c] + t]]++;
+    // Extend-add chunks per (height of the parent, rank of the child).
+    std::vector<int2> ch;
+    struct Chunks {
+        int64_t height, at, count;  // into ch
+    };
+    std::vector<Chunks> chunks;
+    for (int64_t h = 1; h <= height_; ++h) {
+        int maxrank = -1;
+        for (int64_t p : levels_[h]) maxrank = std::max<int>(maxrank, (int)(cptr[p + 1] - cptr[p]) - 1);
+        for (int r = 0; r <= maxrank; ++r) {
+            Chunks c{h, (int64_t)ch.size(), 0};
+            for (int64_t p : levels_[h]) {
+                if (cptr[p + 1] - cptr[p] <= r) continue;
+                const int64_t cc = clist[cptr[p] + r];
+                const int64_t mu = m_[cc] - k_[cc];
+                const int64_t parts = (mu * mu + CHUNK - 1) / CHUNK;
+                for (int64_t q = 0; q < parts; ++q) ch.push_back(int2{(int)cc, (int)q});
+            }
+            c.count = (int64_t)ch.size() - c.at;
+            if (c.count) chunks.push_back(c);
+        }
+    }
+    if (ns_ >= INT_MAX) throw Failure(FEMGPU_ERR_TOO_LARGE, "too many supernodes");
+    // Device arrays.
+    std::vector<int32_t> col2sn(n_);
+    for (int64_t t = 0; t < ns_; ++t)
+        for (int64_t j = S.first[t]; j < S.first[t + 1]; ++j) col2sn[j] = (int32_t)t;
+    perm_.upload(S.perm.data(), n_, s);
+    DevBuf<int64_t> iperm;
+    iperm.upload(S.iperm.data(), n_, s);
+    first_.upload(S.first.data(), ns_ + 1, s);
+    rows_ptr_.upload(S.rows_ptr.data(), ns_ + 1, s);
+    rows_.upload(S.rows.data(), S.rows.size(), s);
+    foff_.upload(foff.data(), ns_, s);
+    host_foff_ = foff;
+    host_first_ = S.first;
+    slot_ptr_.upload(slot_ptr.data(), nrows + 1, s);
+    dst_.upload(dst.data(), nrows, s);
+    slot_.alloc(std::max<size_t>(1, slot_ptr[nrows]));
+    DevBuf<uint32_t> relind;
+    DevBuf<int64_t> relind_off, small_list, parent;
+    DevBuf<int2> chunk;
+    relind.upload(rel.data(), rel.size(), s);
+    relind_off.upload(roff.data(), ns_, s);
+    small_list.upload(sl.data(), sl.size(), s);
+    chunk.upload(ch.data(), ch.size(), s);
+    parent.upload(S.parent.data(), ns_, s);
+    DevBuf<int32_t> dcol2sn;
+    dcol2sn.upload(col2sn.data(), n_, s);
+    fronts_.alloc(fv);
+    FG_CUDA(cudaMemsetAsync(fronts_.p, 0, fv * sizeof(double), s));
+    y_.alloc(n_);
+    xs_.alloc(n_);
+    DevBuf<int64_t> aptr;
+    DevBuf<uint32_t> aidx;
+    DevBuf<double> aval, diag0(n_);
+    aptr.upload(a.ptr.data(), n_ + 1, s);
+    aidx.upload(a.idx.data(), a.nnz(), s);
+    aval.upload(a.val.data(), a.nnz(), s);
+    DevBuf<unsigned long long> status(1);
+    FG_CUDA(cudaMemsetAsync(status.p, 0xff, sizeof(unsigned long long), s));
+    const Fronts fr{first_.p, rows_ptr_.p, rows_.p, foff_.p, fronts_.p};
+    k_assemble_fronts<<<blocks_for(n_, TH), TH, 0, s>>>(n_, perm_.p, iperm.p, aptr.p, aidx.p,
+                                                       aval.p, dcol2sn.p, fr, diag0.p);
     FG_CHECK_LAUNCH();
-    DenseBatchWork w;
-    triangular_inverse_batch(ns, ls, ws, &w, s);
-    winv_off_.upload(off.data(), ns_, s);
-    FG_CUDA(cudaStreamSynchronize(s));
+    const size_t smem = (size_t)SMALL_ROWS * SMALL_ROWS * sizeof(double);
+    FG_CUDA(cudaFuncSetAttribute(k_front_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)smem));
+    size_t ci = 0;
+    for (int64_t h = 0; h <= height_; ++h) {
+        for (; ci < chunks.size() && chunks[ci].height == h; ++ci)
+            k_extend_add<<<(unsigned)chunks[ci].count, TH, 0, s>>>(
+                chunk.p + chunks[ci].at, fr, parent.p, relind.p, relind_off.p);
+        const int64_t ns_small = small_at[h + 1] - small_at[h];
+        if (ns_small > 0) {
+            int mmax = 0;
+            for (int64_t t : small[h]) mmax = std::max<int>(mmax, (int)m_[t]);
+            k_front_small<<<(unsigned)ns_small, TH, (size_t)mmax * mmax * sizeof(double), s>>>(
+                small_list.p + small_at[h], fr, diag0.p, status.p);
+        }
+        for (int64_t t : large[h])
+            dense_partial_cholesky(fronts_.p + foff[t], m_[t], k_[t], diag0.p + S.first[t],
+                                   S.first[t], status.p, s);
+        FG_CHECK_LAUNCH();
+    }
+    unsigned long long bad = fetch(status.p, s);
+    if (bad != ~0ull) {
+        const int64_t j = (int64_t)bad;
+        const double d = fetch(diag0.p + j, s);
+        char buf[320];
+        std::snprintf(buf, sizeof buf,
+                      "the matrix is not positive definite: the pivot of column %lld is 0 or less "
+                      "to the precision of the arithmetic (its diagonal is %s)",
+                      (long long)S.perm[j], rust_exp_shortest(d).c_str());
+        throw Failure(FEMGPU_ERR_NOT_SPD, buf);
+    }
+    pack(s);
 }
 
-void SparseFactor::solve(const double* b, double* x, cudaStream_t s) {
+// The supernodes' G panels from the fronts, which are then freed.
+void SparseFactor::pack(cudaStream_t s) {
+    std::vector<int64_t> goff(ns_), gld(ns_);
+    int64_t total = 0;
+    std::vector<int64_t> small, large;
+    for (int64_t t = 0; t < ns_; ++t) {
+        gld[t] = (m_[t] + 3) & ~(int64_t)3;  // columns start on 32-byte sectors
+        goff[t] = total;
+        total += gld[t] * k_[t];
+        (k_[t] <= INV_SMALL ? small : large).push_back(t);
+    }
+    g_.alloc(std::max<int64_t>(1, total));
+    DevBuf<int64_t> dgoff, dgld, dsmall;
+    dgoff.upload(goff.data(), ns_, s);
+    dgld.upload(gld.data(), ns_, s);
     const Fronts fr{first_.p, rows_ptr_.p, rows_.p, foff_.p, fronts_.p};
-    k_permute_in<<<blocks_for(n_, TH), TH, 0, s>>>(n_, perm_.p, b, y_.p);
+    if (!small.empty()) {
+        dsmall.upload(small.data(), small.size(), s);
+        k_small_inverse<<<(unsigned)small.size(), 128, 0, s>>>(dsmall.p, fr, dgoff.p, dgld.p,
+                                                               g_.p);
+        FG_CHECK_LAUNCH();
+    }
+    // The larger ones' W by the batched triangular inverse, a bounded number at a time.
+    constexpr size_t AT_ONCE = 4096;
+    constexpr int64_t VALUES_AT_ONCE = (int64_t)1 << 27;
+    for (size_t at = 0, end; at < large.size(); at = end) {
+        int64_t kk = 0, kmax = 0;
+        for (end = at; end < large.size() && end - at < AT_ONCE; ++end) {
+            const int64_t k = k_[large[end]];
+            if (end > at && kk + k * k > VALUES_AT_ONCE) break;
+            kk += k * k;
+            kmax = std::max(kmax, k);
+        }
+        DevBuf<double> lc(kk), wc(kk);
+        std::vector<BlockCopy> bc;
+        std::vector<GTile> tiles;
+        std::vector<int64_t> n;
+        std::vector<double*> ls, ws;
+        int64_t off = 0;
+        for (size_t e = at; e < end; ++e) {
+            const int64_t t = large[e];
+            const double* F = fronts_.p + host_foff_[t];
+            bc.push_back({F, lc.p + off, m_[t], k_[t]});
+            n.push_back(k_[t]);
+            ls.push_back(lc.p + off);
+            ws.push_back(wc.p + off);
+            for (int64_t r0 = 0; r0 < gld[t]; r0 += 64)
+                for (int64_t c0 = 0; c0 < k_[t]; c0 += 64)
+                    tiles.push_back(GTile{F, wc.p + off, g_.p + goff[t], m_[t], k_[t], gld[t],
+                                          (int)r0, (int)c0});
+            off += k_[t] * k_[t];
+        }
+        DevBuf<BlockCopy> dbc;
+        dbc.upload(bc.data(), bc.size(), s);
+        k_copy_blocks<<<dim3((unsigned)blocks_for(kmax * kmax, TH, 256), (unsigned)bc.size()), TH,
+                        0, s>>>(dbc.p);
+        FG_CHECK_LAUNCH();
+        DenseBatchWork w;
+        triangular_inverse_batch(n, ls, ws, &w, s);
+        DevBuf<GTile> dt;
+        dt.upload(tiles.data(), tiles.size(), s);
+        k_large_panel<<<(unsigned)tiles.size(), TH, 0, s>>>(dt.p);
+        FG_CHECK_LAUNCH();
+        FG_CUDA(cudaStreamSynchronize(s));
+    }
+    // The tasks of each level.
+    std::vector<SolveBlock> fb, bb;
+    std::vector<SolveTask> ft, bt;
+    forward_at_.assign(1, 0);
+    backward_at_.assign(1, 0);
+    // Tasks of 16, 4 and 1 warps go to blocks of their own kind; the long ones first.
+    auto flush = [&](std::vector<SolveTask> (&kind)[3], std::vector<SolveTask>& tasks,
+                     std::vector<SolveBlock>& blocks) {
+        for (int q = 0; q < 3; ++q) {
+            const int warps = q == 0 ? 16 : q == 1 ? 4 : 1, per = SOLVE_WARPS / warps;
+            for (size_t e = 0; e < kind[q].size(); e += per)
+                blocks.push_back(SolveBlock{(int)(tasks.size() + e),
+                                            (int)std::min<size_t>(per, kind[q].size() - e), warps});
+            tasks.insert(tasks.end(), kind[q].begin(), kind[q].end());
+        }
+    };
     for (int64_t h = 0; h <= height_; ++h) {
-        const int64_t cnt = level_at_[h + 1] - level_at_[h];
-        if (cnt)
-            k_forward<<<(unsigned)cnt, TH, 0, s>>>(level_list_.p + level_at_[h], fr, zoff_.p,
-                                                   child_ptr_.p, child_.p, relind_.p,
-                                                   relind_off_.p, work_.p, y_.p, winv_off_.p,
-                                                   winv_.p, tmp_.p);
+        std::vector<SolveTask> fk[3], bk[3];
+        for (int64_t t : levels_[h]) {
+            SolveTask q{};
+            q.g = goff[t];
+            q.z = host_zoff_[t];
+            q.j0 = host_first_[t];
+            q.ld = (int)gld[t];
+            q.m = (int)m_[t];
+            q.k = (int)k_[t];
+            // Forward: at most 32 entries of G per thread up to 128 columns (a warp alone up to
+            // 32, 4 warps up to 128), 16 warps above.
+            const int fq = k_[t] <= 32 ? 2 : k_[t] <= 128 ? 1 : 0;
+            for (int64_t r = 0; r < m_[t]; r += 32) {
+                q.at = (int)r;
+                fk[fq].push_back(q);
+            }
+            // Backward: 1 warp takes 4 columns of up to 128 rows, 4 warps 2 columns each of up
+            // to 512, 16 warps 1 column each above: 16 to 32 entries of G per thread.
+            const int bq = m_[t] <= ZCAP - 4 ? 2 : m_[t] <= 4 * ZCAP - 4 ? 1 : 0;
+            const int step = bq == 2 ? COLS_1 : bq == 1 ? 4 * COLS_4 : 16;
+            for (int64_t c = 0; c < k_[t]; c += step) {
+                q.at = (int)c;
+                q.cols = (int)std::min<int64_t>(step, k_[t] - c);
+                bk[bq].push_back(q);
+            }
+        }
+        flush(fk, ft, fb);
+        flush(bk, bt, bb);
+        forward_at_.push_back((int64_t)fb.size());
+        backward_at_.push_back((int64_t)bb.size());
     }
-    for (int64_t h = height_; h >= 0; --h) {
-        const int64_t cnt = level_at_[h + 1] - level_at_[h];
-        if (cnt)
-            k_backward<<<(unsigned)cnt, TH, 0, s>>>(level_list_.p + level_at_[h], fr, zoff_.p,
-                                                    work_.p, y_.p, winv_off_.p, winv_.p,
-                                                    tmp_.p);
-    }
-    k_permute_out<<<blocks_for(n_, TH), TH, 0, s>>>(n_, perm_.p, y_.p, x);
-    FG_CHECK_LAUNCH();
+    forward_blocks_.upload(fb.data(), fb.size(), s);
+    backward_blocks_.upload(bb.data(), bb.size(), s);
+    forward_tasks_.upload(ft.data(), ft.size(), s);
+    backward_tasks_.upload(bt.data(), bt.size(), s);
+    FG_CUDA(cudaStreamSynchronize(s));
+    fronts_.release();
 }
+
+template <class TB, class TX>
+void SparseFactor::solve(const TB* b, TX* x, bool pdl, cudaStream_t s) {
+    for (int64_t h = 0; h <= height_; ++h)
+        launch(pdl, k_sparse_forward<TB>, (int)(forward_at_[h + 1] - forward_at_[h]), SOLVE_TH, s,
+               forward_blocks_.p + forward_at_[h], forward_tasks_.p, g_.p, slot_ptr_.p, dst_.p,
+               perm_.p, b, slot_.p, y_.p);
+    for (int64_t h = height_; h >= 0; --h)
+        launch(pdl, k_sparse_backward<TX>, (int)(backward_at_[h + 1] - backward_at_[h]), SOLVE_TH,
+               s, backward_blocks_.p + backward_at_[h], backward_tasks_.p, g_.p, rows_.p, perm_.p,
+               y_.p, xs_.p, x);
+}
+template void SparseFactor::solve<double, double>(const double*, double*, bool, cudaStream_t);
+template void SparseFactor::solve<float, float>(const float*, float*, bool, cudaStream_t);
 
 size_t SparseFactor::solve_launches() const {
-    size_t c = 2;
-    for (int64_t h = 0; h <= height_; ++h)
-        if (level_at_[h + 1] > level_at_[h]) c += 2;
-    return c;
+    return 2 * (size_t)(height_ + 1);
 }
 
 size_t SparseFactor::bytes() const {
-    return fronts_.bytes() + work_.bytes() + y_.bytes() + perm_.bytes() + first_.bytes() +
-           rows_ptr_.bytes() + rows_.bytes() + foff_.bytes() + zoff_.bytes() +
-           child_ptr_.bytes() + child_.bytes() + relind_.bytes() + relind_off_.bytes() +
-           small_list_.bytes() + level_list_.bytes() + chunk_.bytes() + winv_.bytes() +
-           tmp_.bytes() + winv_off_.bytes();
+    return fronts_.bytes() + g_.bytes() + y_.bytes() + xs_.bytes() + slot_.bytes() +
+           slot_ptr_.bytes() + dst_.bytes() + perm_.bytes() + first_.bytes() +
+           rows_ptr_.bytes() + rows_.bytes() + foff_.bytes() + forward_blocks_.bytes() +
+           backward_blocks_.bytes() + forward_tasks_.bytes() + backward_tasks_.bytes();
 }
 
 std::string SparseFactor::describe() const {
     char buf[256];
-    int64_t nl = 0, mmax = 0;
-    for (const auto& l : large_) nl += (int64_t)l.size();
+    int64_t mmax = 0;
     for (int64_t m : m_) mmax = std::max(mmax, m);
     std::snprintf(buf, sizeof buf,
                   "sparse multifrontal factor: %lld supernodes, %lld levels, %lld fronts above %d "
                   "rows (largest %lld), L entries %llu, flops %.3g, front values %zu\n",
-                  (long long)ns_, (long long)height_ + 1, (long long)nl, SMALL_ROWS,
+                  (long long)ns_, (long long)height_ + 1, (long long)large_fronts_, SMALL_ROWS,
                   (long long)mmax, (unsigned long long)entries_, flops_, front_values_);
     return buf;
 }

@@ -18,8 +18,13 @@
 // A pivot at or below PIVOT = 1e-10 of the column's diagonal of A (cholesky.rs:22, 176-181) is
 // recorded (the smallest column; every front with no failed descendant is still checked, so
 // this is the reference's first failing column) and the factor fails with the reference's text.
-// The solves run level by level too: forward, 1 block per supernode adding its children's
-// contributions in order; backward from the root down.
+// Then the fronts give way to the form of the solves: each supernode's G = [W; -L21 W] with
+// W = L11^-1 (m_s x k_s), so that a supernode's step is 1 product in either direction and splits
+// over as many blocks as it has rows (forward) or columns (backward). The solves run level by
+// level: forward up the tree, backward from the root down. The products round as W does, not as
+// a substitution: on the direct solves of the test systems the true residuals stay those of the
+// substitution (4.1e-11 against 4.3e-11 on a 36,300-unknown P2 beam, 1.4e-15 on a 32^3 heat
+// cube).
 #pragma once
 #include <string>
 #include <vector>
@@ -30,19 +35,27 @@
 
 namespace femgpu {
 
+// A part of a supernode's step in the solves: its panel G (offset g, m rows, k columns, leading
+// dimension ld), where its rows (z) and columns (j0) start, and the part: 32 rows from `at`
+// (forward), or `cols` columns from `at` (backward).
+struct SolveTask {
+    int64_t g, z, j0;
+    int ld, m, k, at, cols, pad;
+};
+// A block's tasks: `count` from `task`, each with `warps` of the block's 16 warps.
+struct SolveBlock {
+    int task, count, warps;
+};
+
 class SparseFactor {
    public:
     // Analyses and factors `a` (host CSR, both triangles) in the nested dissection order of the
     // unknowns' coordinates `xyz` (3 per unknown).
     void factor(const HostCsr& a, const double* xyz, cudaStream_t s);
-    // x = A^-1 b, device arrays of n values (x may not alias b).
-    void solve(const double* b, double* x, cudaStream_t s);
-    // Keeps W = L11^-1 of the diagonal block of each supernode of at least `min_cols` columns,
-    // so that the solves take its triangles by 2 products (fully parallel) instead of column by
-    // column. The products round as W does, not as the substitution: on the direct solves of
-    // the test systems the true residuals stay those of the substitution (4.1e-11 against
-    // 4.3e-11 on a 36,300-unknown P2 beam, 1.4e-15 on a 32^3 heat cube).
-    void invert_blocks(int64_t min_cols, cudaStream_t s);
+    // x = A^-1 b in FP64, device arrays of n values (x may not alias b; both double, or both float
+    // and converted on the way). `pdl`: programmatic dependent launches.
+    template <class TB, class TX>
+    void solve(const TB* b, TX* x, bool pdl, cudaStream_t s);
     int64_t n() const { return n_; }
     // The kernels that 1 solve launches.
     size_t solve_launches() const;
@@ -51,32 +64,28 @@ class SparseFactor {
     uint64_t entries() const { return entries_; }
 
    private:
-    int64_t n_ = 0, ns_ = 0, height_ = 0;
+    void pack(cudaStream_t s);
+
+    int64_t n_ = 0, ns_ = 0, height_ = 0, large_fronts_ = 0;
     uint64_t entries_ = 0;
     double flops_ = 0.0;
     size_t front_values_ = 0;
-    // Per supernode (device): first column, row list, front offset, children.
-    DevBuf<int64_t> perm_, first_, rows_ptr_, foff_, zoff_, child_ptr_, child_;
-    DevBuf<uint32_t> rows_, relind_;
-    DevBuf<int64_t> relind_off_;
-    DevBuf<double> fronts_, work_, y_;
-    // invert_blocks: the inverses end to end, each supernode's offset into them (-1: none), and
-    // a scratch vector of n values.
-    DevBuf<double> winv_, tmp_;
-    DevBuf<int64_t> winv_off_;
-    // The level schedule (host): the supernodes of each height, small and large fronts apart,
-    // and the extend-add chunks per (height, child rank).
-    std::vector<std::vector<int64_t>> small_, large_;
-    std::vector<int64_t> m_, k_;  // rows and columns of each supernode (host)
-    DevBuf<int64_t> small_list_, level_list_;
-    std::vector<int64_t> small_at_, level_at_;  // offsets into the lists per height
-    struct Chunks {
-        int height, rank;
-        int64_t at, count;  // into chunk_
-    };
-    std::vector<Chunks> chunks_;
-    DevBuf<int2> chunk_;  // (child, first entry / 4096)
-    std::vector<int64_t> host_first_, host_foff_;
+    // Per supernode (device): first column, row list, front offset.
+    DevBuf<int64_t> perm_, first_, rows_ptr_, foff_;
+    DevBuf<uint32_t> rows_;
+    DevBuf<double> fronts_;  // until the factor is packed
+    // The G panels end to end; the forward solution and the backward one (both in the
+    // elimination order); the children's updates (slots) with each row's first slot and the
+    // slot that each update row writes in its parent.
+    DevBuf<double> g_, y_, xs_, slot_;
+    DevBuf<uint32_t> slot_ptr_, dst_;
+    DevBuf<SolveBlock> forward_blocks_, backward_blocks_;
+    DevBuf<SolveTask> forward_tasks_, backward_tasks_;
+    std::vector<int64_t> forward_at_, backward_at_;  // per height: offsets into the blocks
+    // Host: the supernodes of each height, their rows and columns, and where their rows, columns
+    // and fronts start.
+    std::vector<std::vector<int64_t>> levels_;
+    std::vector<int64_t> m_, k_, host_zoff_, host_first_, host_foff_;
 };
 
 }  // namespace femgpu

@@ -7,9 +7,10 @@
 // with path compression; a postorder of it; the column counts by walking, for each row, its row
 // subtree up the tree from the row's entries (O(entries of L)); fundamental supernodes (a column
 // joins its predecessor when it is that column's only child and their counts differ by 1); the
-// row pattern of each supernode from its own columns' entries and its children's patterns; and
-// the height of each supernode in the supernode tree, which schedules the device's fronts level
-// by level (every child before its parent).
+// row pattern of each supernode from its own columns' entries and its children's patterns; the
+// merging of a supernode with its last child where that stores few zeros (relaxed supernodes,
+// Ashcraft and Grimes 1989); and the height of each supernode in the supernode tree, which
+// schedules the device's fronts level by level (every child before its parent).
 #pragma once
 #include <cstdint>
 #include <vector>

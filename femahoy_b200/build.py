@@ -41,6 +41,7 @@ UNITS = [
     ("sparse_direct.cu", []),
     ("dense_eigen.cu", []),
     ("dense_factor.cu", []),
+    ("spd_inverse.cu", []),
     ("offsets.cu", []),
     ("extrude.cu", ["-fmad=false"]),
     ("boxgrid.cu", ["-fmad=false"]),

@@ -6,6 +6,7 @@
 
 #include "dense_factor.cuh"
 #include "rust_format.hpp"
+#include "spd_inverse.cuh"
 
 namespace femgpu {
 namespace {
@@ -193,12 +194,6 @@ __device__ __forceinline__ void gemm_sub_body(double* __restrict__ C, int64_t ld
         }
 }
 
-__global__ void __launch_bounds__(TH)
-    k_gemm_sub(double* __restrict__ C, int64_t ldc, const double* __restrict__ A, int64_t lda,
-               const double* __restrict__ B, int64_t ldb, int64_t M, int64_t N, int kb) {
-    gemm_sub_body(C, ldc, A, lda, B, ldb, M, N, kb, blockIdx.x, blockIdx.y);
-}
-
 // Rows [b0, b0 + kb) of W for its columns 0..ncols: W_b = L_bb^-1 W_b (the block's triangle in
 // shared memory), 1 thread per column, the column's 32 values in registers.
 __device__ __forceinline__ void trsm_rows_body(double* __restrict__ W,
@@ -222,12 +217,6 @@ __device__ __forceinline__ void trsm_rows_body(double* __restrict__ W,
 #pragma unroll
     for (int i = 0; i < PANEL; ++i)
         if (i < kb) W[(b0 + i) + c * n] = y[i];
-}
-
-__global__ void __launch_bounds__(ROWS_TH)
-    k_trsm_rows(double* __restrict__ W, const double* __restrict__ L, int64_t n, int64_t b0,
-                int kb, int64_t ncols) {
-    trsm_rows_body(W, L, n, b0, kb, ncols, blockIdx.x);
 }
 
 // X = W^T W (W lower triangular, column-major n x n): 1 block per 64 x 64 tile on or below the
@@ -267,13 +256,8 @@ __device__ __forceinline__ void gram_lower_body(const double* __restrict__ W, in
         }
 }
 
-__global__ void __launch_bounds__(TH)
-    k_gram_lower(const double* __restrict__ W, int64_t n, double* __restrict__ X) {
-    gram_lower_body(W, n, X, blockIdx.x);
-}
-
-// The dense lower triangle of a host CSR's device copy, and its diagonal.
-__global__ void k_scatter_dense(int64_t n, const int64_t* __restrict__ ptr,
+// The dense lower triangle of a host CSR's device copy (leading dimension ld), and its diagonal.
+__global__ void k_scatter_dense(int64_t n, int64_t ld, const int64_t* __restrict__ ptr,
                                 const uint32_t* __restrict__ idx, const double* __restrict__ val,
                                 double* __restrict__ M, double* __restrict__ diag) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
@@ -282,16 +266,10 @@ __global__ void k_scatter_dense(int64_t n, const int64_t* __restrict__ ptr,
         for (int64_t e = ptr[i]; e < ptr[i + 1]; ++e) {
             const int64_t j = idx[e];
             if (j == i) d = val[e];
-            if (j >= i) M[j + i * n] = val[e];  // column i, row j (symmetric)
+            if (j >= i) M[j + i * ld] = val[e];  // column i, row j (symmetric)
         }
         diag[i] = d;
     }
-}
-
-__global__ void k_identity(int64_t n, double* __restrict__ W) {
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n * n;
-         t += (int64_t)gridDim.x * blockDim.x)
-        W[t] = (t % n == t / n) ? 1.0 : 0.0;
 }
 
 // ---------------------------------------------------------------- many systems at once
@@ -502,7 +480,7 @@ void dense_partial_cholesky(double* F, int64_t m, int64_t k, const double* diag0
 
 void dense_inverse(const HostCsr& a, double* inv, DenseWork* w, cudaStream_t s,
                    std::vector<std::pair<const char*, double>>* stages) {
-    const int64_t n = a.n;
+    const int64_t n = a.n, ld = spd_padded(n);
     auto t0 = std::chrono::steady_clock::now();
     auto stage = [&](const char* name) {
         if (!stages) return;
@@ -516,8 +494,9 @@ void dense_inverse(const HostCsr& a, double* inv, DenseWork* w, cudaStream_t s,
         if (b.count < count) b.alloc(count);
     };
     fit(w->diag, n);
-    fit(w->L, n * n);
-    fit(w->W, n * n);
+    fit(w->L, ld * ld);
+    fit(w->W, ld * ld);
+    fit(w->pair, SPD_PAIR);
     if (!w->status.p) w->status.alloc(1);
     double* L = w->L.p;
     double* W = w->W.p;
@@ -525,12 +504,12 @@ void dense_inverse(const HostCsr& a, double* inv, DenseWork* w, cudaStream_t s,
     w->ptr.upload(a.ptr.data(), n + 1, s);
     w->idx.upload(a.idx.data(), a.nnz(), s);
     w->val.upload(a.val.data(), a.nnz(), s);
-    FG_CUDA(cudaMemsetAsync(L, 0, (size_t)n * n * sizeof(double), s));
-    k_scatter_dense<<<blocks_for(n, TH), TH, 0, s>>>(n, w->ptr.p, w->idx.p, w->val.p, L,
+    FG_CUDA(cudaMemsetAsync(L, 0, (size_t)ld * ld * sizeof(double), s));
+    k_scatter_dense<<<blocks_for(n, TH), TH, 0, s>>>(n, ld, w->ptr.p, w->idx.p, w->val.p, L,
                                                      w->diag.p);
     FG_CUDA(cudaMemsetAsync(w->status.p, 0xff, sizeof(unsigned long long), s));
-    dense_partial_cholesky(L, n, n, w->diag.p, 0, w->status.p, s);
-    stage("factor");
+    spd_factor(n, L, W, w->diag.p, w->pair.p, w->status.p, s);
+    stage("factor and L^-1");
     const unsigned long long bad = fetch(w->status.p, s);
     if (bad != ~0ull) {
         const double d = fetch(w->diag.p + bad, s);
@@ -541,24 +520,7 @@ void dense_inverse(const HostCsr& a, double* inv, DenseWork* w, cudaStream_t s,
                       bad, rust_exp_shortest(d).c_str());
         throw Failure(FEMGPU_ERR_NOT_SPD, buf);
     }
-    // W = L^-1 by block rows of 32: each block's triangle solve, then the rows below updated.
-    k_identity<<<blocks_for(n * n, TH), TH, 0, s>>>(n, W);
-    for (int64_t b0 = 0; b0 < n; b0 += PANEL) {
-        const int kb = (int)std::min<int64_t>(PANEL, n - b0);
-        const int64_t ncols = b0 + kb;
-        k_trsm_rows<<<(unsigned)((ncols + ROWS_TH - 1) / ROWS_TH), ROWS_TH, 0, s>>>(W, L, n, b0,
-                                                                                    kb, ncols);
-        const int64_t rows = n - b0 - kb;
-        if (rows > 0) {
-            dim3 grid((unsigned)((rows + TILE - 1) / TILE), (unsigned)((ncols + TILE - 1) / TILE));
-            k_gemm_sub<<<grid, TH, 0, s>>>(W + b0 + kb, n, L + (b0 + kb) + b0 * n, n, W + b0, n,
-                                           rows, ncols, kb);
-        }
-    }
-    stage("L^-1");
-    const int64_t T = (n + TILE - 1) / TILE;
-    k_gram_lower<<<(unsigned)(T * (T + 1) / 2), TH, 0, s>>>(W, n, inv);
-    FG_CHECK_LAUNCH();
+    spd_gram(n, W, inv, s);
     stage("W^T W");
 }
 

@@ -1,11 +1,12 @@
 // Dense Cholesky factors and inverses on the device, in FP64 on the tensor cores.
 //
-// The panels of a factor are 32 columns: the diagonal block is factored in shared memory by 1
-// block, which then solves the panel's rows below it; the trailing matrix takes the rank-32
-// update in 64 x 64 tiles of mma.sync m8n8k4 f64 products. The inverse of an SPD matrix is
-// W^T W with W = L^-1, formed by a blocked forward substitution (32 rows at a time, each block's
-// triangle in shared memory, the rest of the rows updated by the same tiled products) and a
-// tiled product W^T W. Pivots at or below 1e-10 of their column's diagonal of A fail
+// One matrix alone is inverted in 128-column blocks (spd_inverse.cuh). The partial factors of the
+// sparse solver's fronts and the batched inverses go by panels of 32 columns: the diagonal block
+// is factored in shared memory by 1 block, the panel's rows below it are solved a thread each;
+// the trailing matrix takes the rank-32 update in 64 x 64 tiles of mma.sync m8n8k4 f64 products.
+// A batched inverse is W^T W with W = L^-1, formed by a blocked forward substitution (32 rows at
+// a time, each block's triangle in shared memory, the rest of the rows updated by the same tiled
+// products) and a tiled product W^T W. Pivots at or below 1e-10 of their column's diagonal of A fail
 // (cholesky.rs:22, 173-181): the smallest such column is recorded in `status`.
 #pragma once
 #include <cstdint>
@@ -37,7 +38,7 @@ void dense_inverse(const HostCsr& a, DevBuf<double>* inv, cudaStream_t s,
 struct DenseWork {
     DevBuf<int64_t> ptr;
     DevBuf<uint32_t> idx;
-    DevBuf<double> val, diag, L, W;
+    DevBuf<double> val, diag, L, W, pair;
     DevBuf<unsigned long long> status;
 };
 // The same into `inv` (n x n, the caller's), with the buffers of `w`; returns with the work

@@ -42,6 +42,7 @@ UNITS = [
     ("dense_eigen.cu", []),
     ("dense_factor.cu", []),
     ("spd_inverse.cu", []),
+    ("pool.cu", []),
     ("offsets.cu", []),
     ("extrude.cu", ["-fmad=false"]),
     ("boxgrid.cu", ["-fmad=false"]),

@@ -16,28 +16,33 @@ static thread_local std::string g_last_error;
 
 void set_last_error(const std::string& s) { g_last_error = s; }
 
+// A stream for calls that have no handle (assembly, utilities).
+static thread_local cudaStream_t g_util_stream = nullptr;
+static cudaStream_t util_stream() {
+    if (!g_util_stream)
+        FG_CUDA(cudaStreamCreateWithFlags(&g_util_stream, cudaStreamNonBlocking));
+    return g_util_stream;
+}
+
+// A call that failed leaves nothing in flight on its thread's stream.
 template <class F>
 static int guarded(F f) {
+    int code;
     try {
         f();
         return FEMGPU_OK;
     } catch (const Failure& e) {
         set_last_error(e.what());
-        return e.code;
+        code = e.code;
     } catch (const std::bad_alloc&) {
         set_last_error("out of host memory");
-        return FEMGPU_ERR_TOO_LARGE;
+        code = FEMGPU_ERR_TOO_LARGE;
     } catch (const std::exception& e) {
         set_last_error(e.what());
-        return FEMGPU_ERR_INVALID;
+        code = FEMGPU_ERR_INVALID;
     }
-}
-
-// A stream for calls that have no handle (assembly, utilities).
-static cudaStream_t util_stream() {
-    static thread_local cudaStream_t s = nullptr;
-    if (!s) FG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    return s;
+    if (g_util_stream) cudaStreamSynchronize(g_util_stream);
+    return code;
 }
 
 static void require(bool ok, const char* what) {
@@ -70,6 +75,7 @@ static int assemble_impl(int kind, int mode, size_t npoints, const double* xyz, 
         require(npoints > 0 && nel > 0, "an empty mesh");
         require(xyz && nodes && coef, "a null mesh array");
         cudaStream_t s = util_stream();
+        PoolScope pool(s);
         int nn = kind >= FEMGPU_HEX8_HEAT ? 8 : (kind >= FEMGPU_P2_ELASTIC ? 10 : 4);
         int nc = (kind == FEMGPU_P1_HEAT || kind == FEMGPU_HEX8_HEAT)
                      ? 3
@@ -113,6 +119,7 @@ int femgpu_pattern(size_t n, size_t nel, int m, const uint32_t* elements, femgpu
     return guarded([&] {
         require(out && elements && m > 0 && n > 0, "invalid pattern arguments");
         cudaStream_t s = util_stream();
+        PoolScope pool(s);
         DevBuf<uint32_t> de;
         de.upload(elements, (size_t)m * nel, s);
         Incidence inc;
@@ -129,6 +136,7 @@ int femgpu_colour(size_t n, size_t nel, int m, const uint32_t* elements, uint32_
     return guarded([&] {
         require(elements && colour && ncolours && m > 0, "invalid colouring arguments");
         cudaStream_t s = util_stream();
+        PoolScope pool(s);
         DevBuf<uint32_t> de;
         de.upload(elements, (size_t)m * nel, s);
         Incidence inc;
@@ -145,6 +153,7 @@ int femgpu_quadratic(size_t ncorner, size_t ntet, const uint32_t* tets, uint32_t
     return guarded([&] {
         require(tets && tets10 && edges && nedges, "a null array");
         cudaStream_t s = util_stream();
+        PoolScope pool(s);
         DevBuf<uint32_t> dt, d10(10 * ntet), de(12 * ntet);
         dt.upload(tets, 4 * ntet, s);
         int64_t ne = quadratic((int64_t)ncorner, (int64_t)ntet, dt.p, d10.p, de.p, s);
@@ -167,6 +176,7 @@ int femgpu_csr_download(const femgpu_csr* a, int64_t* ptr, uint32_t* idx, double
     return guarded([&] {
         require(a != nullptr, "null matrix");
         cudaStream_t s = util_stream();
+        PoolScope pool(s);
         if (ptr) a->m.ptr.download(ptr, a->m.n + 1, s);
         if (idx) a->m.idx.download(idx, a->m.nnz, s);
         if (val) a->m.val.download(val, a->m.nnz, s);
@@ -181,6 +191,7 @@ int femgpu_csr_upload(size_t n, const int64_t* ptr, const uint32_t* idx, const d
         require(ptr[0] == 0, "ptr[0] must be 0");
         for (size_t i = 0; i < n; ++i) require(ptr[i + 1] >= ptr[i], "ptr must not decrease");
         cudaStream_t s = util_stream();
+        PoolScope pool(s);
         auto* h = new femgpu_csr;
         h->m.n = (int64_t)n;
         h->m.nnz = ptr[n];
@@ -197,6 +208,7 @@ int femgpu_csr_submatrix(const femgpu_csr* a, const int64_t* keep, size_t nkeep,
     return guarded([&] {
         require(a && keep && out, "null argument");
         cudaStream_t s = util_stream();
+        PoolScope pool(s);
         DevBuf<int64_t> dk;
         dk.upload(keep, nkeep, s);
         auto* h = new femgpu_csr;
@@ -215,6 +227,7 @@ int femgpu_csr_mul(const femgpu_csr* a, const double* x, double* y) {
     return guarded([&] {
         require(a && x && y, "null argument");
         cudaStream_t s = util_stream();
+        PoolScope pool(s);
         DevBuf<double> dx, dy(a->m.n);
         dx.upload(x, a->m.n, s);
         csr_mul(a->m, dx.p, dy.p, s);
@@ -228,6 +241,7 @@ int femgpu_reduced_rhs(const femgpu_csr* a, const double* load, const double* t,
     return guarded([&] {
         require(a && load && t && free && out, "null argument");
         cudaStream_t s = util_stream();
+        PoolScope pool(s);
         DevBuf<double> dl, dt, dout(nfree);
         DevBuf<int64_t> df;
         dl.upload(load, a->m.n, s);
@@ -342,6 +356,7 @@ int femgpu_hex_elements(size_t count, const double* keys, double* matrices) {
     return guarded([&] {
         require(count > 0 && keys && matrices, "null or empty cell keys");
         cudaStream_t s = util_stream();
+        PoolScope pool(s);
         DevBuf<double> dk, dt(576 * count);
         dk.upload(keys, 12 * count, s);
         hex_elements(dk.p, (int64_t)count, dt.p, s);
@@ -378,6 +393,7 @@ int femgpu_coarse_matrix(const femgpu_csr* a, const femgpu_unknowns* u,
         require(u->kind == FEMGPU_UNKNOWNS_GRID, "coarse matrices need grid unknowns");
         require(level >= 1, "level 1 is the first coarse level");
         cudaStream_t s = util_stream();
+        PoolScope pool(s);
         HostLevel lv = host_level(u, a->m.n);
         HostCells stored, first = host_cells(cells, u);
         const int threads = host_threads();

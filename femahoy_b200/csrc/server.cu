@@ -140,6 +140,7 @@ class Server {
     bool make_room(size_t bytes) {
         // Least recently used at the back of the list.
         auto k = lru_.end();
+        bool freed = false;
         while (used_ + bytes > budget_ && k != lru_.begin()) {
             --k;
             auto it = resident_.find(*k);
@@ -149,7 +150,9 @@ class Server {
             ++k;
             lru_.erase(dead);
             resident_.erase(it);
+            freed = true;
         }
+        if (freed) pool_trim();
         return used_ + bytes <= budget_;
     }
 

@@ -2029,16 +2029,17 @@ SolverImpl::SolverImpl() {
     FG_CUDA(cudaStreamCreateWithFlags(&s_, cudaStreamNonBlocking));
     FG_CUDA(cudaEventCreate(&ev0_));
     FG_CUDA(cudaEventCreate(&ev1_));
-    partial_.alloc(2 * 1024);
-    counter_.alloc(1);
-    counter_.zero(s_);
-    sc_.alloc(1);
-    done_zero_.alloc(1);
-    done_zero_.zero(s_);
     FG_CUDA(cudaMallocHost(&h_sc_, sizeof(Scalars)));
     FG_CUDA(cudaHostAlloc(&h_cancel_, sizeof(int), cudaHostAllocMapped));
     *h_cancel_ = 0;
     FG_CUDA(cudaHostGetDevicePointer(&d_cancel_, h_cancel_, 0));
+    PoolScope pool(s_);
+    partial_.alloc(2 * 1024);
+    sc_.alloc(1);
+    counter_.alloc(1);
+    done_zero_.alloc(1);
+    counter_.zero(s_);
+    done_zero_.zero(s_);
 }
 
 SolverImpl::~SolverImpl() {
@@ -2170,6 +2171,7 @@ static std::vector<double> unknown_xyz(const femgpu_unknowns& u, int64_t n) {
 
 void SolverImpl::create(const DevCsr& a, const femgpu_unknowns& u, int method,
                         const femgpu_crossover& c, const Options& o, const HostCells* cells) {
+    PoolScope pool(s_);  // every buffer of the setup is made, used and freed on the stream
     opt_ = o;
     pdl_ = o.pdl != 0;
     n_ = a.n;

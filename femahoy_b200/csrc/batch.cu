@@ -1502,7 +1502,7 @@ void BatchImpl::create(const std::vector<const DevCsr*>& a,
         for (auto& h : Hs) parts.push_back(h.mats[0]);
         DevCsr f;
         combine(parts, &f, s_);
-        if (opt_.format == 0 && make_bsell3_device<double>(f, &f3ptr_, &f3col_, &f3val_, s_))
+        if (opt_.format == 0 && make_bsell3_device<double>(f, &f3ptr_, &f3col_, &f3val_, nullptr, s_))
             fine3_ = true;
         else
             make_sell<double>(f, 32, &A64_, s_);
@@ -1576,7 +1576,7 @@ void BatchImpl::build_levels(std::vector<SystemHierarchy>& H, std::vector<BatchL
             }
             DevCsr d;
             combine(mats, &d, s_);
-            if (opt_.format == 0 && make_bsell3_device<T>(d, &L.b3ptr, &L.b3col, &L.b3val, s_))
+            if (opt_.format == 0 && make_bsell3_device<T>(d, &L.b3ptr, &L.b3col, &L.b3val, nullptr, s_))
                 L.block3 = true;
             else
                 make_sell<T>(d, 32, &L.A, s_);

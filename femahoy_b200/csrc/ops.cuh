@@ -57,6 +57,7 @@ struct MarchGeom {
 
 template <class T>
 struct SellOp {
+    static constexpr int ROWS = 1;
     SellView<T> v;
     __device__ __forceinline__ int64_t threads() const { return v.nslices * v.C; }
     __device__ __forceinline__ bool valid(int64_t g) const { return g < v.n; }
@@ -85,6 +86,7 @@ __device__ __forceinline__ TA stencil_apply(const StencilView<T>& v, int i,
 
 template <class T>
 struct StencilOp {
+    static constexpr int ROWS = 1;
     StencilView<T> v;
     __device__ __forceinline__ int64_t threads() const { return v.n; }
     __device__ __forceinline__ bool valid(int64_t) const { return true; }
@@ -124,6 +126,7 @@ struct SellRefOp {
 // past either end are predicated off and count 0.
 template <class T, int K>
 struct StencilOpK {
+    static constexpr int ROWS = 1;
     StencilView<T> v;
     __device__ __forceinline__ int64_t threads() const { return v.n; }
     __device__ __forceinline__ bool valid(int64_t) const { return true; }
@@ -166,6 +169,7 @@ struct StencilViewH {
 
 template <int KC>
 struct StencilOpH {
+    static constexpr int ROWS = 1;
     StencilViewH v;
     __device__ __forceinline__ int64_t threads() const { return v.n; }
     __device__ __forceinline__ bool valid(int64_t) const { return true; }

@@ -161,6 +161,17 @@ static bool make_stencil(const DevCsr& d, Operator<T>* out, cudaStream_t s) {
     return true;
 }
 
+// The threads per block row of a 3x3-block operator of `nb` block rows: more where the rows alone
+// leave the device short of loads in flight. Measured (us per finest FP32 step, FP64 product):
+// 672,400 rows 141 / 230 with 1, 149 / 224 with 2; 219,209 uneven rows 66 / 101, 58 / 78 and 67 /
+// 100 with 4; 34,680 rows 16.2 / 15.7 with 2, 13.5 / 17.9 with 4; the 10,000 to 40,000 rows of the
+// coarser levels took 13 to 23 us less per iteration with 4 than with 1.
+template <class T>
+static int block3_split(int64_t nb) {
+    if (sizeof(T) == 8) return nb >= 25'000 ? 2 : 4;
+    return nb >= 250'000 ? 1 : nb >= 60'000 ? 2 : 4;
+}
+
 template <class T>
 void make_operator(const DevCsr& d, int C, bool allow, Operator<T>* out, cudaStream_t s) {
     if (allow && make_stencil<T>(d, out, s)) return;
@@ -169,8 +180,9 @@ void make_operator(const DevCsr& d, int C, bool allow, Operator<T>* out, cudaStr
     out->nnz = d.nnz;
     // Elasticity levels (node-major unknowns, grid order): the 3x3-block form, 40 bytes per 9
     // FP32 entries instead of 72.
-    if (allow && make_bsell3_device<T>(d, &out->b3ptr, &out->b3col, &out->b3val, s)) {
+    if (allow && make_bsell3_device<T>(d, &out->b3ptr, &out->b3col, &out->b3val, &out->b3row, s)) {
         out->block3 = true;
+        out->split = block3_split<T>(d.n / 3);
         return;
     }
     make_sell<T>(d, C, &out->sell, s);
@@ -194,8 +206,12 @@ static void with_op(const Operator<T>& op, F&& f) {
             return;
         }
     }
-    if (op.block3)
-        f(Block3Op<T>{op.b3view(), (int)op.n});
+    if (op.block3 && op.split == 4)
+        f(Block3Op<T, 4>{op.b3view(), (int)op.n});
+    else if (op.block3 && op.split == 2)
+        f(Block3Op<T, 2>{op.b3view(), (int)op.n});
+    else if (op.block3)
+        f(Block3Op<T, 1>{op.b3view(), (int)op.n});
     else if (!op.stencil)
         f(SellOp<T>{op.sell.view()});
     else if (op.unrolled && op.K == 8)
@@ -216,6 +232,29 @@ static void with_op(const Operator<T>& op, F&& f) {
 // 64-bit grid-stride loop around the same product, the finest stencil step took 1.6 times as
 // long on B200.
 __device__ __forceinline__ int row_of_thread() { return (int)(blockIdx.x * blockDim.x + threadIdx.x); }
+
+// What a kernel may load of an operator before it waits for the kernel before it (a 3x3-block
+// operator's first blocks; nothing of the others), and the rows of thread t: f(row, (A x)[row]).
+// Every thread of a block calls them.
+struct NoHead {};
+template <class Op>
+__device__ __forceinline__ auto op_head(const Op& A, int t) {
+    if constexpr (Op::ROWS == 3)
+        return A.head(t);
+    else
+        return NoHead{};
+}
+template <class TA, class Op, class Head, class TX, class F>
+__device__ __forceinline__ void op_rows(const Op& A, const Head& head, int t,
+                                        const TX* __restrict__ x, F&& f) {
+    if constexpr (Op::ROWS == 3) {
+        A.template apply<TA>(head, t, x, f);
+    } else {
+        if (t >= A.threads()) return;
+        const TA ax = A.template apply<TA>(t, x);
+        if (A.valid(t)) f(t, ax);
+    }
+}
 
 // ------------------------------------------------------------------ V-cycle rows
 // The work of 1 row of each V-cycle step, shared by the separate kernels below and by the fused
@@ -242,7 +281,19 @@ __device__ __forceinline__ T cheb_update(T bi, T ax, T di, T dprev, T c1, T c2) 
     return fmadd(c1 * di, r, c2 * dprev);
 }
 
-// A Chebyshev step: r = b - A x_in, d = c2 d + c1 D^-1 r, x_out = x_in + d.
+// A Chebyshev step: r = b - A x_in, d = c2 d + c1 D^-1 r, x_out = x_in + d, from the row's
+// product ax.
+template <class T, bool COH = false>
+__device__ __forceinline__ void cheb_finish_row(int g, T ax, const T* __restrict__ b,
+                                                const T* __restrict__ xin,
+                                                const T* __restrict__ dinv, T c1, T c2,
+                                                T* __restrict__ d, T* __restrict__ xout) {
+    const T bg = COH ? ldx<true>(b + g) : b[g];
+    const T dd = cheb_update(bg, ax, dinv[g], d[g], c1, c2);
+    d[g] = dd;
+    xout[g] = (COH ? ldx<true>(xin + g) : xin[g]) + dd;
+}
+
 template <class T, class Op, bool COH = false>
 __device__ __forceinline__ void cheb_step_row(const Op& A, int g, const T* __restrict__ b,
                                               const T* __restrict__ xin,
@@ -250,10 +301,7 @@ __device__ __forceinline__ void cheb_step_row(const Op& A, int g, const T* __res
                                               T* __restrict__ d, T* __restrict__ xout) {
     T ax = A.template apply<T>(g, xin);
     if (!A.valid(g)) return;
-    const T bg = COH ? ldx<true>(b + g) : b[g];
-    const T dd = cheb_update(bg, ax, dinv[g], d[g], c1, c2);
-    d[g] = dd;
-    xout[g] = (COH ? ldx<true>(xin + g) : xin[g]) + dd;
+    cheb_finish_row<T, COH>(g, ax, b, xin, dinv, c1, c2, d, xout);
 }
 
 template <class T, class Op, bool COH = false>
@@ -393,11 +441,13 @@ __global__ void __launch_bounds__(TH)
     k_cheb_step(Op A, const T* __restrict__ b, const T* __restrict__ xin,
                 const T* __restrict__ dinv, T c1, T c2, T* __restrict__ d, T* __restrict__ xout,
                 const int* __restrict__ done) {
+    const int t = row_of_thread();
+    const auto head = op_head(A, t);
     pdl_wait();
     if (*done) return;
-    const int g = row_of_thread();
-    if (g >= A.threads()) return;
-    cheb_step_row(A, g, b, xin, dinv, c1, c2, d, xout);
+    op_rows<T>(A, head, t, xin, [&](int g, T ax) {
+        cheb_finish_row(g, ax, b, xin, dinv, c1, c2, d, xout);
+    });
 }
 
 // r = b - A x
@@ -405,11 +455,11 @@ template <class T, class Op>
 __global__ void __launch_bounds__(TH)
     k_residual(Op A, const T* __restrict__ b, const T* __restrict__ x, T* __restrict__ r,
                const int* __restrict__ done) {
+    const int t = row_of_thread();
+    const auto head = op_head(A, t);
     pdl_wait();
     if (*done) return;
-    const int g = row_of_thread();
-    if (g >= A.threads()) return;
-    residual_row(A, g, b, x, r);
+    op_rows<T>(A, head, t, x, [&](int g, T ax) { r[g] = b[g] - ax; });
 }
 
 // ------------------------------------------------------------------ 2 rows per thread
@@ -1419,19 +1469,17 @@ template <class Op>
 __global__ void __launch_bounds__(TH)
     k_pcg_residual(Op A, const double* __restrict__ b, const double* __restrict__ x,
                    double* __restrict__ r, float* __restrict__ r32, double* __restrict__ partial) {
+    const int t = row_of_thread();
+    const auto head = op_head(A, t);
     pdl_wait();
     double bb = 0, rr = 0;
-    const int g = row_of_thread();
-    if (g < A.threads()) {
-        double ax = A.template apply<double>(g, x);
-        if (A.valid(g)) {
-            double bi = b[g], ri = bi - ax;
-            r[g] = ri;
-            if (r32) r32[g] = (float)ri;
-            bb = bi * bi;
-            rr = ri * ri;
-        }
-    }
+    op_rows<double>(A, head, t, x, [&](int g, double ax) {
+        double bi = b[g], ri = bi - ax;
+        r[g] = ri;
+        if (r32) r32[g] = (float)ri;
+        bb += bi * bi;
+        rr += ri * ri;
+    });
     block_partial(bb, rr, partial);
 }
 
@@ -1449,17 +1497,15 @@ template <class Op>
 __global__ void __launch_bounds__(TH)
     k_pcg_spmv_pq(Op A, const double* __restrict__ p, double* __restrict__ q,
                   double* __restrict__ partial, const Scalars* __restrict__ sc) {
+    const int t = row_of_thread();
+    const auto head = op_head(A, t);
     pdl_wait();
     if (sc->done) return;
     double pq = 0;
-    const int g = row_of_thread();
-    if (g < A.threads()) {
-        double ap = A.template apply<double>(g, p);
-        if (A.valid(g)) {
-            q[g] = ap;
-            pq = p[g] * ap;
-        }
-    }
+    op_rows<double>(A, head, t, p, [&](int g, double ap) {
+        q[g] = ap;
+        pq += p[g] * ap;
+    });
     block_partial(pq, 0.0, partial);
 }
 
@@ -1618,15 +1664,12 @@ __global__ void __launch_bounds__(TH)
     k_power_step(Op A, const double* __restrict__ v, const double* __restrict__ dg,
                  double* __restrict__ w, double* __restrict__ partial) {
     double vav = 0, vdv = 0;
-    const int g = row_of_thread();
-    if (g < A.threads()) {
-        double av = A.template apply<double>(g, v);
-        if (A.valid(g)) {
-            vav = v[g] * av;
-            vdv = v[g] * dg[g] * v[g];
-            w[g] = av / dg[g];
-        }
-    }
+    const int t = row_of_thread();
+    op_rows<double>(A, op_head(A, t), t, v, [&](int g, double av) {
+        vav += v[g] * av;
+        vdv += v[g] * dg[g] * v[g];
+        w[g] = av / dg[g];
+    });
     block_partial(vav, vdv, partial);
 }
 
@@ -2190,7 +2233,10 @@ void SolverImpl::create(const DevCsr& a, const femgpu_unknowns& u, int method,
         make_sell<double>(a_, C, &A64_, s_);
     }
     // The block partials of the reductions: 1 block per 256 rows of the largest operator.
-    partial_.alloc(2 * (size_t)row_blocks(std::max<int64_t>(a.n, A64_.nslices * A64_.C) + 64));
+    // (or per 256 threads of a 3x3-block operator, up to 4 per block row).
+    partial_.alloc(2 * (size_t)row_blocks(
+                           std::max<int64_t>({a.n, A64_.nslices * A64_.C, 4 * (a.n / 3 + B3C)}) +
+                           64));
     x_.alloc(n_);
     r_.alloc(n_);
     p_.alloc(n_);

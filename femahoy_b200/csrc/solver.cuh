@@ -55,12 +55,13 @@ struct Operator {
     DevBuf<__half> hcoef;
     float hscale = 1.0f;
     DevBuf<int64_t> b3ptr;
-    DevBuf<uint32_t> b3col;
+    DevBuf<uint32_t> b3col, b3row;
     DevBuf<T> b3val;
-    BSell3View<T> b3view() const { return {n / 3, b3ptr.p, b3col.p, b3val.p}; }
+    int split = 1;  // threads per block row (Block3Op)
+    BSell3View<T> b3view() const { return {n / 3, b3ptr.p, b3col.p, b3val.p, b3row.p}; }
     int64_t threads() const {
         if (stencil) return n;
-        if (block3) return 3 * ((n / 3 + B3C - 1) / B3C) * B3C;
+        if (block3) return (n / 3 + B3C - 1) / B3C * B3C * split;
         return sell.nslices * sell.C;
     }
     StencilView<T> sview() const {
@@ -84,7 +85,7 @@ struct Operator {
     }
     size_t bytes() const {
         return sell.bytes() + coef.bytes() + hcoef.bytes() + b3ptr.bytes() + b3col.bytes() +
-               b3val.bytes();
+               b3row.bytes() + b3val.bytes();
     }
     // The bytes one product reads and writes, each value once: the stored coefficients (and
     // indices), x and y.

@@ -262,13 +262,13 @@ __device__ __forceinline__ void op_rows(const Op& A, const Head& head, int t,
 // form, whose right sides and iterates it wrote itself before a grid-wide barrier, read through
 // ldx<true> (L2, coherent) instead of the read-only path.
 
-// The first Chebyshev step from x = 0: d = c1 D^-1 b, x = d.
+// The first Chebyshev step from x = 0: d = c1 D^-1 b, x = d (d null: the next step reads x).
 template <class T, bool COH = false>
 __device__ __forceinline__ void cheb_first_row(int i, const T* __restrict__ b,
                                                const T* __restrict__ dinv, T c1,
                                                T* __restrict__ d, T* __restrict__ x) {
     T v = c1 * dinv[i] * (COH ? ldx<true>(b + i) : b[i]);
-    d[i] = v;
+    if (d) d[i] = v;
     x[i] = v;
 }
 
@@ -283,15 +283,19 @@ __device__ __forceinline__ T cheb_update(T bi, T ax, T di, T dprev, T c1, T c2) 
 
 // A Chebyshev step: r = b - A x_in, d = c2 d + c1 D^-1 r, x_out = x_in + d, from the row's
 // product ax.
+// `din` null: c2 = 0, the first step of a sweep. `dout` null: the sweep's last step, whose d no
+// step reads. Returns x_out.
 template <class T, bool COH = false>
-__device__ __forceinline__ void cheb_finish_row(int g, T ax, const T* __restrict__ b,
-                                                const T* __restrict__ xin,
-                                                const T* __restrict__ dinv, T c1, T c2,
-                                                T* __restrict__ d, T* __restrict__ xout) {
+__device__ __forceinline__ T cheb_finish_row(int g, T ax, const T* __restrict__ b,
+                                             const T* __restrict__ xin,
+                                             const T* __restrict__ dinv, T c1, T c2,
+                                             const T* din, T* dout, T* __restrict__ xout) {
     const T bg = COH ? ldx<true>(b + g) : b[g];
-    const T dd = cheb_update(bg, ax, dinv[g], d[g], c1, c2);
-    d[g] = dd;
-    xout[g] = (COH ? ldx<true>(xin + g) : xin[g]) + dd;
+    const T dd = cheb_update(bg, ax, dinv[g], din ? din[g] : (T)0, c1, c2);
+    if (dout) dout[g] = dd;
+    const T x = (COH ? ldx<true>(xin + g) : xin[g]) + dd;
+    xout[g] = x;
+    return x;
 }
 
 template <class T, class Op, bool COH = false>
@@ -301,7 +305,7 @@ __device__ __forceinline__ void cheb_step_row(const Op& A, int g, const T* __res
                                               T* __restrict__ d, T* __restrict__ xout) {
     T ax = A.template apply<T>(g, xin);
     if (!A.valid(g)) return;
-    cheb_finish_row<T, COH>(g, ax, b, xin, dinv, c1, c2, d, xout);
+    cheb_finish_row<T, COH>(g, ax, b, xin, dinv, c1, c2, d, d, xout);
 }
 
 template <class T, class Op, bool COH = false>
@@ -439,14 +443,14 @@ __global__ void k_cheb_first(int64_t n, const T* __restrict__ b, const T* __rest
 template <class T, class Op>
 __global__ void __launch_bounds__(TH)
     k_cheb_step(Op A, const T* __restrict__ b, const T* __restrict__ xin,
-                const T* __restrict__ dinv, T c1, T c2, T* __restrict__ d, T* __restrict__ xout,
-                const int* __restrict__ done) {
+                const T* __restrict__ dinv, T c1, T c2, const T* din, T* dout,
+                T* __restrict__ xout, const int* __restrict__ done) {
     const int t = row_of_thread();
     const auto head = op_head(A, t);
     pdl_wait();
     if (*done) return;
     op_rows<T>(A, head, t, xin, [&](int g, T ax) {
-        cheb_finish_row(g, ax, b, xin, dinv, c1, c2, d, xout);
+        cheb_finish_row(g, ax, b, xin, dinv, c1, c2, din, dout, xout);
     });
 }
 
@@ -999,7 +1003,7 @@ __global__ void __launch_bounds__(TH)
     const T s = offset_row<T, KC>(M, i, in);
     out[i] = s;
     const T v = c1 * dinv[i] * s;
-    d[i] = v;
+    if (d) d[i] = v;
     x[i] = v;
 }
 
@@ -1454,6 +1458,25 @@ __global__ void __launch_bounds__(FIN_TH) k_finish(const double* __restrict__ pa
 }
 
 // ------------------------------------------------------------------ PCG kernels (FP64)
+// The start of a solve: |b|, |r|, and whether there is nothing to iterate (b = 0, or x solves it).
+struct FinStart {
+    Scalars* sc;
+    __device__ bool skip() const { return false; }
+    __device__ void operator()(double bb, double rr) const {
+        sc->bb = bb;
+        sc->norm_b = sqrt(bb);
+        sc->rr = rr;
+        sc->done = bb == 0.0 || sqrt(rr) / sqrt(bb) <= sc->tol;
+    }
+};
+
+// The true residual at the end of a solve.
+struct FinTruth {
+    Scalars* sc;
+    __device__ bool skip() const { return false; }
+    __device__ void operator()(double, double rr) const { sc->truth = rr; }
+};
+
 struct FinResidual0 {
     Scalars* sc;
     __device__ bool skip() const { return false; }
@@ -1558,21 +1581,24 @@ __global__ void __launch_bounds__(TH)
 
 struct FinUpdate {
     Scalars* sc;
-    double tol;
     __device__ bool skip() const { return sc->done; }
     __device__ void operator()(double rr, double) const {
         sc->rr = rr;
         sc->iters += 1;
         // multigrid.rs:722-723: |r| / |b| <= tol, on the updated residual.
-        if (sqrt(rr) / sc->norm_b <= tol) sc->done = 1;
+        if (sqrt(rr) / sc->norm_b <= sc->tol) sc->done = 1;
     }
 };
 
-// x += alpha p, r -= alpha q (multigrid.rs:742-745), with the partial sums of r.r.
+// x += alpha p, r -= alpha q (multigrid.rs:742-745), with the partial sums of r.r; also the FP32
+// copy of r (mixed form), and with `xfirst` the V-cycle's first smoothing step on the new r (T the
+// cycle's type, the bits of k_cheb_first): r is at hand here, and a launch less.
+template <class T>
 __global__ void __launch_bounds__(TH)
     k_pcg_update(int64_t n, double* __restrict__ x, double* __restrict__ r,
                  const double* __restrict__ p, const double* __restrict__ q,
-                 float* __restrict__ r32, double* __restrict__ partial,
+                 float* __restrict__ r32, const T* __restrict__ dinv, T c1,
+                 T* __restrict__ dfirst, T* __restrict__ xfirst, double* __restrict__ partial,
                  const Scalars* __restrict__ sc) {
     pdl_wait();
     if (sc->done) return;
@@ -1584,6 +1610,11 @@ __global__ void __launch_bounds__(TH)
         double ri = r[i] - alpha * q[i];
         r[i] = ri;
         if (r32) r32[i] = (float)ri;
+        if (xfirst) {
+            const T v = c1 * dinv[i] * (T)ri;
+            if (dfirst) dfirst[i] = v;
+            xfirst[i] = v;
+        }
         rr = ri * ri;
     }
     block_partial(rr, 0.0, partial);
@@ -1608,6 +1639,29 @@ struct FinDots {
     }
 };
 
+// The V-cycle's last smoothing step with the partial sums of r.z and z.q on the z it computes (q
+// null: r.z alone), which saves reading z again and a launch.
+template <class T, class Op>
+__global__ void __launch_bounds__(TH)
+    k_cheb_step_dots(Op A, const T* __restrict__ b, const T* __restrict__ xin,
+                     const T* __restrict__ dinv, T c1, T c2, const T* din,
+                     T* __restrict__ xout, const double* __restrict__ r,
+                     const double* __restrict__ q, double* __restrict__ partial,
+                     const Scalars* __restrict__ sc) {
+    const int t = row_of_thread();
+    const auto head = op_head(A, t);
+    pdl_wait();
+    if (sc->done) return;
+    double rz = 0, zq = 0;
+    op_rows<T>(A, head, t, xin, [&](int g, T ax) {
+        const double z =
+            (double)cheb_finish_row(g, ax, b, xin, dinv, c1, c2, din, (T*)nullptr, xout);
+        rz += r[g] * z;
+        if (q) zq += z * q[g];
+    });
+    block_partial(rz, zq, partial);
+}
+
 template <class TZ>
 __global__ void __launch_bounds__(TH)
     k_pcg_dots(int64_t n, const double* __restrict__ r, const TZ* __restrict__ z,
@@ -1625,26 +1679,25 @@ __global__ void __launch_bounds__(TH)
     block_partial(rz, zq, partial);
 }
 
-// p = z + beta p (multigrid.rs:749-751); p = z on the first call.
+// p = z + beta p (multigrid.rs:749-751); p = z on the first call. Within the solve's graph
+// (`cancel` not null) also the loop's condition: go on unless the solve converged, reached its
+// iteration limit, broke down (a NaN residual) or was cancelled (multigrid.rs:721-738).
 template <class TZ>
 __global__ void k_pcg_p(int64_t n, const TZ* __restrict__ z, double* __restrict__ p,
-                        const Scalars* sc, int init) {
+                        const Scalars* sc, int init, cudaGraphConditionalHandle loop,
+                        const volatile int* cancel) {
     pdl_wait();
+    const int i = row_of_thread();
+    if (i == 0 && cancel) {
+        const double rr = sc->rr;
+        const bool go = !sc->done && sc->iters < sc->max_iter && rr == rr && !*cancel &&
+                        !sc->bulk_timeout;
+        cudaGraphSetConditional(loop, go ? 1u : 0u);
+    }
     if (sc->done) return;
     const double beta = sc->beta;
-    const int i = row_of_thread();
     if (i >= n) return;
     p[i] = init ? (double)z[i] : (double)z[i] + beta * p[i];
-}
-
-// The end of a device-side PCG iteration: continue unless the solve converged, reached its
-// iteration limit, broke down (a NaN residual) or was cancelled (multigrid.rs:721-738, in the
-// same order of tests).
-__global__ void k_loop_control(cudaGraphConditionalHandle h, const Scalars* sc,
-                               const volatile int* cancel) {
-    double rr = sc->rr;
-    bool go = !sc->done && sc->iters < sc->max_iter && rr == rr && !*cancel && !sc->bulk_timeout;
-    cudaGraphSetConditional(h, go ? 1u : 0u);
 }
 
 // ------------------------------------------------------------------ power iteration
@@ -2072,7 +2125,8 @@ SolverImpl::SolverImpl() {
     FG_CUDA(cudaStreamCreateWithFlags(&s_, cudaStreamNonBlocking));
     FG_CUDA(cudaEventCreate(&ev0_));
     FG_CUDA(cudaEventCreate(&ev1_));
-    FG_CUDA(cudaMallocHost(&h_sc_, sizeof(Scalars)));
+    FG_CUDA(cudaMallocHost(&h_sc_, 2 * sizeof(Scalars)));
+    h_init_ = h_sc_ + 1;
     FG_CUDA(cudaHostAlloc(&h_cancel_, sizeof(int), cudaHostAllocMapped));
     *h_cancel_ = 0;
     FG_CUDA(cudaHostGetDevicePointer(&d_cancel_, h_cancel_, 0));
@@ -2228,15 +2282,9 @@ void SolverImpl::create(const DevCsr& a, const femgpu_unknowns& u, int method,
     FG_CUDA(cudaMemcpyAsync(a_.idx.p, a.idx.p, a_.idx.bytes(), cudaMemcpyDeviceToDevice, s_));
     FG_CUDA(cudaMemcpyAsync(a_.val.p, a.val.p, a_.val.bytes(), cudaMemcpyDeviceToDevice, s_));
     int C = o.sell_c ? o.sell_c : 32;
-    {
-        PhaseTimer t{this, "outer SELL", s_};
-        make_sell<double>(a_, C, &A64_, s_);
-    }
-    // The block partials of the reductions: 1 block per 256 rows of the largest operator.
-    // (or per 256 threads of a 3x3-block operator, up to 4 per block row).
-    partial_.alloc(2 * (size_t)row_blocks(
-                           std::max<int64_t>({a.n, A64_.nslices * A64_.C, 4 * (a.n / 3 + B3C)}) +
-                           64));
+    // The block partials of the reductions: 1 block per 256 rows of an operator (SELL rows padded
+    // to slices of at most 64), or per 256 threads of a 3x3-block operator, up to 4 per block row.
+    partial_.alloc(2 * (size_t)row_blocks(std::max<int64_t>(a.n, 4 * (a.n / 3 + B3C)) + 64));
     x_.alloc(n_);
     r_.alloc(n_);
     p_.alloc(n_);
@@ -2278,7 +2326,14 @@ void SolverImpl::create(const DevCsr& a, const femgpu_unknowns& u, int method,
         direct = entries <= c.entries && (c.flat || flops <= c.flops * (double)a.n);
     }
     direct_ = direct;
+    // The matrix exactly, for the true residual and the direct method, where the operator of PCG
+    // does not hold every entry itself (a stencil takes the lower triangle from the upper one).
+    auto exact_matrix = [&] {
+        PhaseTimer t{this, "outer SELL", s_};
+        make_sell<double>(a_, C, &A64_, s_);
+    };
     if (direct) {
+        exact_matrix();
         // A small system takes the dense inverse; a larger one the sparse multifrontal factor in
         // the reference's order.
         if (a.n <= DENSE_DIRECT) {
@@ -2297,6 +2352,7 @@ void SolverImpl::create(const DevCsr& a, const femgpu_unknowns& u, int method,
         tune_operator(&op64_, opt_.stencil, s_);
         if (!opt_.sell_c) tune_sell(a_, &op64_, s_);
     }
+    if (op64_.stencil) exact_matrix();
     if (u.kind == FEMGPU_UNKNOWNS_GRID) {
         HostLevel lv;
         for (int d = 0; d < 3; ++d) lv.planes[d].assign(u.planes[d], u.planes[d] + u.nplanes[d]);
@@ -2743,9 +2799,23 @@ void SolverImpl::build_multigrid(HostLevel level, const HostRect* pfirst,
     }
 }
 
-// A Chebyshev step and the residual of level L: by tiles when the autotuner chose them.
+// Whether a level's steps run as the kernels of 1 row (or block row) per thread.
 template <class T>
-void SolverImpl::enqueue_step(MgLevel<T>& L, const T* b, const T* xin, T c1, T c2, T* xout) {
+static bool row_kernels(const Operator<T>& A) {
+    return !A.bulk && !A.march && !A.pair;
+}
+// Where the first smoothing step of L leaves d: nowhere if the next step takes it from x.
+template <class T>
+static T* first_d(MgLevel<T>& L) {
+    return row_kernels(L.A) ? nullptr : L.d.p;
+}
+
+// A Chebyshev step and the residual of level L: by tiles when the autotuner chose them. `din`,
+// `dout`: see cheb_finish_row (the tiles, pairs and planes update L.d in place). `dots`: also the
+// partial sums of r.z and z.q.
+template <class T>
+void SolverImpl::enqueue_step(MgLevel<T>& L, const T* b, const T* xin, T c1, T c2, const T* din,
+                              T* dout, T* xout, const Dots* dots) {
     const int* done = &sc_.p->done;
     if constexpr (std::is_same<T, float>::value) {
         if (L.A.bulk) {
@@ -2771,8 +2841,14 @@ void SolverImpl::enqueue_step(MgLevel<T>& L, const T* b, const T* xin, T c1, T c
         return;
     }
     with_op(L.A, [&](auto op) {
-        launch(pdl_, k_cheb_step<T, decltype(op)>, row_blocks(L.A.threads()), TH, s_, op, b,
-               xin, L.dinv.p, c1, c2, L.d.p, xout, done);
+        const int grid = row_blocks(L.A.threads());
+        if (dots)
+            launch(pdl_, k_cheb_step_dots<T, decltype(op)>, grid, TH, s_, op, b, xin,
+                   (const T*)L.dinv.p, c1, c2, din, xout, (const double*)r_.p, dots->q,
+                   partial_.p, (const Scalars*)sc_.p);
+        else
+            launch(pdl_, k_cheb_step<T, decltype(op)>, grid, TH, s_, op, b, xin,
+                   (const T*)L.dinv.p, c1, c2, din, dout, xout, done);
     });
 }
 
@@ -2807,7 +2883,8 @@ void SolverImpl::enqueue_residual(MgLevel<T>& L, const T* b, const T* x) {
 }
 
 template <class T>
-const T* SolverImpl::enqueue_vcycle(Hierarchy<T>& H, size_t l, const T* b, bool started) {
+const T* SolverImpl::enqueue_vcycle(Hierarchy<T>& H, size_t l, const T* b, bool started,
+                                    const Dots* dots) {
     const int* done = &sc_.p->done;
     if (l == H.levels.size() && H.sparse) {
         // The sparse coarsest factor's 2 triangular solves in FP64 (the right side and the
@@ -2887,12 +2964,17 @@ const T* SolverImpl::enqueue_vcycle(Hierarchy<T>& H, size_t l, const T* b, bool 
     T* xb = L.xb.p;
     int deg = (int)L.c1.size();
     std::string tag = "L" + std::to_string(l) + " ";
+    // The kernels of 1 row or block row per thread read d only where a step needs it: after the
+    // first step d is x itself, and no step reads the last one's d.
+    const bool in_place = !row_kernels(L.A);
     if (!started) {
-        launch(pdl_, k_cheb_first<T>, gb, TH, s_, n, b, L.dinv.p, (T)L.c1[0], L.d.p, xa, done);
+        launch(pdl_, k_cheb_first<T>, gb, TH, s_, n, b, L.dinv.p, (T)L.c1[0], first_d(L), xa, done);
         mark(tag + "smooth (first, no product)");
     }
     for (int k = 1; k < deg; ++k) {
-        enqueue_step(L, b, xa, (T)L.c1[k], (T)L.c2[k], xb);
+        enqueue_step(L, b, xa, (T)L.c1[k], (T)L.c2[k],
+                     k == 1 && !in_place ? (const T*)xa : (const T*)L.d.p,
+                     k + 1 < deg || in_place ? L.d.p : nullptr, xb);
         mark(tag + "smooth pre");
         std::swap(xa, xb);
     }
@@ -2909,10 +2991,10 @@ const T* SolverImpl::enqueue_vcycle(Hierarchy<T>& H, size_t l, const T* b, bool 
         const auto v = L.Ro.view();
         if (v.K == 27)
             launch(pdl_, k_restrict_first<T, 27>, row_blocks(L.nc), TH, s_, v, (const T*)L.r.p,
-                   bc, (const T*)N.dinv.p, (T)N.c1[0], N.d.p, N.xa.p, done);
+                   bc, (const T*)N.dinv.p, (T)N.c1[0], first_d(N), N.xa.p, done);
         else
             launch(pdl_, k_restrict_first<T, 0>, row_blocks(L.nc), TH, s_, v, (const T*)L.r.p,
-                   bc, (const T*)N.dinv.p, (T)N.c1[0], N.d.p, N.xa.p, done);
+                   bc, (const T*)N.dinv.p, (T)N.c1[0], first_d(N), N.xa.p, done);
     } else if (L.Ro.ok) {
         launch_transfer(L.Ro, (const T*)L.r.p, bc, 0, done, s_, pdl_);
     } else {
@@ -2930,8 +3012,11 @@ const T* SolverImpl::enqueue_vcycle(Hierarchy<T>& H, size_t l, const T* b, bool 
         launch(pdl_, k_prolong<T>, gb, TH, s_, n, L.pptr.p, L.pidx.p, L.pval.p, ec, xa, done);
     mark(tag + "prolong + correct");
     for (int k = 0; k < deg; ++k) {
-        enqueue_step(L, b, xa, (T)L.c1[k], (T)L.c2[k], xb);
-        mark(tag + "smooth post");
+        const bool last = k + 1 == deg;
+        enqueue_step(L, b, xa, (T)L.c1[k], (T)L.c2[k],
+                     k > 0 || in_place ? (const T*)L.d.p : nullptr,
+                     !last || in_place ? L.d.p : nullptr, xb, last ? dots : nullptr);
+        mark(tag + (last && dots ? "smooth post, r.z, z.q partials" : "smooth post"));
         std::swap(xa, xb);
     }
     FG_CHECK_LAUNCH();
@@ -2958,71 +3043,156 @@ void SolverImpl::enqueue_spmv_pq() {
     }
 }
 
-void SolverImpl::enqueue_iteration() {
-    int64_t n = n_;
-    launches_ += 7;
+// The V-cycle on r (`started`: its first smoothing step is done), then r.z, z.q and beta, and the
+// new p. `init`: the solve's first cycle (no q yet, p = z).
+template <class T>
+void SolverImpl::enqueue_cycle(Hierarchy<T>& H, const T* r, bool started, bool init) {
     Scalars* sc = sc_.p;
-    bool mixed = opt_.precision == FEMGPU_MIXED;
+    const bool mixed = std::is_same<T, float>::value;
+    const int64_t n = n_;
+    const int nbn = row_blocks(n);
+    // The last smoothing step takes the sums along where it runs row by row.
+    const Dots with{mixed && !init ? q_.p : nullptr};
+    const bool fused = !H.levels.empty() && row_kernels(H.levels[0].A) &&
+                       !(H.tail_from == 0 && tail_on_);
+    const T* z = enqueue_vcycle(H, 0, r, started, fused ? &with : nullptr);
+    int parts = nbn;
+    if (fused) {
+        parts = row_blocks(H.levels[0].A.threads());
+    } else {
+        launch(pdl_, k_pcg_dots<T>, nbn, TH, s_, n, r_.p, z, q_.p, mixed ? 1 : 0, init ? 1 : 0,
+               partial_.p, sc);
+        mark(mixed ? "pcg r.z, z.q partials" : "pcg r.z partials");
+        launches_ += 1;
+    }
+    launch(pdl_, k_finish<FinDots>, 1, FIN_TH, s_, partial_.p, parts,
+           FinDots{sc, mixed ? 1 : 0, init ? 1 : 0});
+    mark("pcg beta");
+    launch(pdl_, k_pcg_p<T>, nbn, TH, s_, n, z, p_.p, sc, init ? 1 : 0, cond_,
+           in_graph_ ? (const volatile int*)d_cancel_ : nullptr);
+    mark("pcg p = z + beta p");
+    FG_CHECK_LAUNCH();
+    launches_ += 2;
+}
+
+// The start of a solve from x: r = b - A x, and the first p.
+void SolverImpl::enqueue_start() {
+    const bool mixed = opt_.precision == FEMGPU_MIXED;
+    FG_CUDA(cudaMemcpyAsync(sc_.p, h_init_, sizeof(Scalars), cudaMemcpyHostToDevice, s_));
+    const int nbq = row_blocks(op64_.threads());
+    with_op(op64_, [&](auto op) {
+        launch(false, k_pcg_residual<decltype(op)>, nbq, TH, s_, op, b_.p, x_.p, r_.p,
+               mixed ? r32_.p : nullptr, partial_.p);
+    });
+    launch(pdl_, k_finish<FinStart>, 1, FIN_TH, s_, partial_.p, nbq, FinStart{sc_.p});
+    FG_CHECK_LAUNCH();
+    launches_ += 2;
+    if (mixed)
+        enqueue_cycle<float>(H32_, r32_.p, false, true);
+    else
+        enqueue_cycle<double>(H64_, r_.p, false, true);
+}
+
+void SolverImpl::enqueue_iteration() {
+    const int64_t n = n_;
+    Scalars* sc = sc_.p;
     const int nbq = row_blocks(op64_.threads()), nbn = row_blocks(n);
     enqueue_spmv_pq();
     mark("pcg q = A p, p.q partials (fp64)");
     launch(pdl_, k_finish<FinPq>, 1, FIN_TH, s_, partial_.p, nbq, FinPq{sc});
     mark("pcg alpha");
-    launch(pdl_, k_pcg_update, nbn, TH, s_, n, x_.p, r_.p, p_.p, q_.p, mixed ? r32_.p : nullptr,
-                                     partial_.p, sc);
-    mark("pcg x, r update, r.r partials");
-    launch(pdl_, k_finish<FinUpdate>, 1, FIN_TH, s_, partial_.p, nbn, FinUpdate{sc, tol});
-    FG_CHECK_LAUNCH();
-    mark("pcg stopping test");
-    if (mixed) {
-        zf_ = enqueue_vcycle<float>(H32_, 0, r32_.p);
-        launch(pdl_, k_pcg_dots<float>, nbn, TH, s_, n, r_.p, zf_, q_.p, 1, 0, partial_.p, sc);
-        mark("pcg r.z, z.q partials");
-        launch(pdl_, k_finish<FinDots>, 1, FIN_TH, s_, partial_.p, nbn, FinDots{sc, 1, 0});
-        mark("pcg beta");
-        launch(pdl_, k_pcg_p<float>, nbn, TH, s_, n, zf_, p_.p, sc, 0);
-        mark("pcg p = z + beta p");
-    } else {
-        zd_ = enqueue_vcycle<double>(H64_, 0, r_.p);
-        launch(pdl_, k_pcg_dots<double>, nbn, TH, s_, n, r_.p, zd_, q_.p, 0, 0, partial_.p, sc);
-        mark("pcg r.z partials");
-        launch(pdl_, k_finish<FinDots>, 1, FIN_TH, s_, partial_.p, nbn, FinDots{sc, 0, 0});
-        mark("pcg beta");
-        launch(pdl_, k_pcg_p<double>, nbn, TH, s_, n, zd_, p_.p, sc, 0);
-        mark("pcg p = z + beta p");
-    }
-    FG_CHECK_LAUNCH();
+    auto rest = [&](auto& H, auto* r, float* r32) {
+        typedef std::remove_pointer_t<decltype(r)> T;
+        // The first smoothing step rides on the update where the cycle starts with one.
+        const bool first = !H.levels.empty() && !(H.tail_from == 0 && tail_on_);
+        MgLevel<T>* L = first ? &H.levels[0] : nullptr;
+        launch(pdl_, k_pcg_update<T>, nbn, TH, s_, n, x_.p, r_.p, p_.p, q_.p, r32,
+               (const T*)(first ? L->dinv.p : nullptr), (T)(first ? L->c1[0] : 0.0),
+               first ? first_d(*L) : nullptr, first ? L->xa.p : nullptr, partial_.p, sc);
+        mark(first ? "pcg x, r update, r.r partials, L0 first smooth"
+                   : "pcg x, r update, r.r partials");
+        launch(pdl_, k_finish<FinUpdate>, 1, FIN_TH, s_, partial_.p, nbn, FinUpdate{sc});
+        FG_CHECK_LAUNCH();
+        mark("pcg stopping test");
+        launches_ += 4;
+        enqueue_cycle<T>(H, r, first, false);
+    };
+    if (opt_.precision == FEMGPU_MIXED)
+        rest(H32_, r32_.p, r32_.p);
+    else
+        rest(H64_, r_.p, (float*)nullptr);
 }
 
-// The whole PCG loop as 1 graph: a WHILE conditional node whose body is 1 iteration followed by
-// k_loop_control, so the device runs iteration after iteration with no host round trip.
-void SolverImpl::build_loop_graph() {
+// The true residual of x, by the operator that holds every entry of the matrix.
+void SolverImpl::enqueue_truth() {
+    const bool sell = op64_.stencil;
+    const int nb = sell ? row_blocks(A64_.nslices * A64_.C) : row_blocks(op64_.threads());
+    if (sell)
+        launch(pdl_, k_pcg_residual<SellOp<double>>, nb, TH, s_, SellOp<double>{A64_.view()},
+               b_.p, x_.p, t_.p, (float*)nullptr, partial_.p);
+    else
+        with_op(op64_, [&](auto op) {
+            launch(pdl_, k_pcg_residual<decltype(op)>, nb, TH, s_, op, b_.p, x_.p, t_.p,
+                   (float*)nullptr, partial_.p);
+        });
+    launch(pdl_, k_finish<FinTruth>, 1, FIN_TH, s_, partial_.p, nb, FinTruth{sc_.p});
+    FG_CHECK_LAUNCH();
+    launches_ += 2;
+    FG_CUDA(cudaMemcpyAsync(h_sc_, sc_.p, sizeof(Scalars), cudaMemcpyDeviceToHost, s_));
+}
+
+// The whole solve as 1 graph: its start, a WHILE conditional node whose body is 1 iteration, and
+// the true residual, so that the device runs from the first residual to the last with no host
+// round trip. (With the start and the true residual as stream launches around the loop's graph, a
+// solve waited for the device 4 times: 118 of the 188 us of the 3,000 unknown cantilever, 155 of
+// 755 us at 110,544 unknowns.)
+void SolverImpl::build_graph() {
     for (;;) {
         const size_t before = launches_;
         try {
             FG_CUDA(cudaGraphCreate(&graph_, 0));
-            FG_CUDA(cudaGraphConditionalHandleCreate(&cond_, graph_, 1,
+            FG_CUDA(cudaGraphConditionalHandleCreate(&cond_, graph_, 0,
                                                      cudaGraphCondAssignDefault));
+            in_graph_ = true;
+            FG_CUDA(cudaStreamBeginCaptureToGraph(s_, graph_, nullptr, nullptr, 0,
+                                                  cudaStreamCaptureModeThreadLocal));
+            enqueue_start();
+            fixed_kernels_ = launches_ - before;
+            cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+            const cudaGraphNode_t* at = nullptr;
+            size_t count = 0;
+            FG_CUDA(cudaStreamGetCaptureInfo(s_, &st, nullptr, nullptr, &at, &count));
+            const std::vector<cudaGraphNode_t> last(at, at + count);
+            cudaGraph_t same = nullptr;
+            FG_CUDA(cudaStreamEndCapture(s_, &same));
             cudaGraphNodeParams cp{};
             cp.type = cudaGraphNodeTypeConditional;
             cp.conditional.handle = cond_;
             cp.conditional.type = cudaGraphCondTypeWhile;
             cp.conditional.size = 1;
             cudaGraphNode_t node;
-            FG_CUDA(cudaGraphAddNode(&node, graph_, nullptr, 0, &cp));
+            FG_CUDA(cudaGraphAddNode(&node, graph_, last.data(), last.size(), &cp));
             cudaGraph_t body = cp.conditional.phGraph_out[0];
+            launches_ = before;
             FG_CUDA(cudaStreamBeginCaptureToGraph(s_, body, nullptr, nullptr, 0,
                                                   cudaStreamCaptureModeThreadLocal));
             enqueue_iteration();
-            k_loop_control<<<1, 1, 0, s_>>>(cond_, sc_.p, d_cancel_);
-            FG_CUDA(cudaStreamEndCapture(s_, &body));
+            FG_CUDA(cudaStreamEndCapture(s_, &same));
+            loop_kernels_ = launches_ - before;
+            launches_ = before;
+            FG_CUDA(cudaStreamBeginCaptureToGraph(s_, graph_, &node, nullptr, 1,
+                                                  cudaStreamCaptureModeThreadLocal));
+            enqueue_truth();
+            FG_CUDA(cudaStreamEndCapture(s_, &same));
+            fixed_kernels_ += launches_ - before;
             FG_CUDA(cudaGraphInstantiate(&exec_, graph_, 0));
-            graph_kernels_ = launches_ - before + 1;
+            in_graph_ = false;
             launches_ = before;
             return;
         } catch (const Failure&) {
             // A capture that failed (a cooperative launch that the graph did not take, for
-            // one) ends here; the loop is captured again with every step its own launch.
+            // one) ends here; the solve is captured again with every step its own launch.
+            in_graph_ = false;
             cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
             cudaStreamIsCapturing(s_, &st);
             if (st != cudaStreamCaptureStatusNone) {
@@ -3061,9 +3231,9 @@ void SolverImpl::set_wait_limit(unsigned polls) {
     graph_ = nullptr;
 }
 
-void SolverImpl::run_device_loop(const volatile int* cancel) {
-    int before = h_sc_->iters;
-    *(volatile int*)h_cancel_ = 0;
+// Runs the solve's graph; *h_sc_ holds the scalars when it returns.
+void SolverImpl::run_graph(const volatile int* cancel) {
+    *(volatile int*)h_cancel_ = cancel && *cancel ? 1 : 0;
     std::atomic<bool> stop{false};
     std::thread watcher;
     if (cancel) {
@@ -3075,13 +3245,30 @@ void SolverImpl::run_device_loop(const volatile int* cancel) {
             }
         });
     }
+    const int before = h_init_->iters;
     cudaError_t e = cudaGraphLaunch(exec_, s_);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h_sc_, sc_.p, sizeof(Scalars), cudaMemcpyDeviceToHost, s_);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s_);
     stop.store(true);
     if (watcher.joinable()) watcher.join();
     FG_CUDA(e);
-    launches_ += graph_kernels_ * (size_t)(h_sc_->iters - before);
+    launches_ += fixed_kernels_ + loop_kernels_ * (size_t)(h_sc_->iters - before);
+}
+
+// The same with every kernel its own launch (option graph = 2).
+void SolverImpl::run_launches(const volatile int* cancel) {
+    auto scalars = [&] {
+        FG_CUDA(cudaMemcpyAsync(h_sc_, sc_.p, sizeof(Scalars), cudaMemcpyDeviceToHost, s_));
+        FG_CUDA(cudaStreamSynchronize(s_));
+    };
+    enqueue_start();
+    scalars();
+    while (!h_sc_->done && h_sc_->iters < h_sc_->max_iter && h_sc_->rr == h_sc_->rr &&
+           !h_sc_->bulk_timeout && !(cancel && *cancel)) {
+        enqueue_iteration();
+        scalars();
+    }
+    enqueue_truth();
+    FG_CUDA(cudaStreamSynchronize(s_));
 }
 
 // Host vectors: b and the start value go straight into the solver's own device vectors and the
@@ -3141,9 +3328,9 @@ void SolverImpl::solve(const double* d_b, double* d_x, const volatile int* cance
     bool mixed = opt_.precision == FEMGPU_MIXED;
     FG_CUDA(cudaEventRecord(ev0_, s_));
     if (d_b != b_.p) FG_CUDA(cudaMemcpyAsync(b_.p, d_b, n * 8, cudaMemcpyDeviceToDevice, s_));
-    Scalars init{};
-    init.max_iter = (int)std::min<size_t>(max_iter, 0x7fffffff);
-    FG_CUDA(cudaMemcpyAsync(sc_.p, &init, sizeof(Scalars), cudaMemcpyHostToDevice, s_));
+    *h_init_ = Scalars{};
+    h_init_->max_iter = (int)std::min<size_t>(max_iter, 0x7fffffff);
+    h_init_->tol = tol;
     femgpu_stats out{};
     launches_ = 0;
     if (direct_) {
@@ -3158,6 +3345,7 @@ void SolverImpl::solve(const double* d_b, double* d_x, const volatile int* cance
             }
         };
         launches_ = 8;
+        FG_CUDA(cudaMemcpyAsync(sc_.p, h_init_, sizeof(Scalars), cudaMemcpyHostToDevice, s_));
         apply(b_.p, x_.p);
         k_pcg_residual<<<row_blocks(A64_.nslices * A64_.C), TH, 0, s_>>>(
             SellOp<double>{A64_.view()}, b_.p, x_.p, r_.p, nullptr, partial_.p);
@@ -3188,76 +3376,48 @@ void SolverImpl::solve(const double* d_b, double* d_x, const volatile int* cance
     }
     // multigrid.rs:692-753
     if (d_x != x_.p) FG_CUDA(cudaMemcpyAsync(x_.p, d_x, n * 8, cudaMemcpyDeviceToDevice, s_));
-    with_op(op64_, [&](auto op) {
-        k_pcg_residual<<<row_blocks(op64_.threads()), TH, 0, s_>>>(
-            op, b_.p, x_.p, r_.p, mixed ? r32_.p : nullptr, partial_.p);
-    });
-    k_finish<<<1, FIN_TH, 0, s_>>>(partial_.p, row_blocks(op64_.threads()), FinResidual0{sc_.p});
-    FG_CHECK_LAUNCH();
-    launches_ += 5;  // this residual and its sum, r.z and its sum, and p = z  // this residual, and r.z and p = z after the first cycle
-    FG_CUDA(cudaMemcpyAsync(h_sc_, sc_.p, sizeof(Scalars), cudaMemcpyDeviceToHost, s_));
-    FG_CUDA(cudaStreamSynchronize(s_));
-    double norm_b = h_sc_->norm_b;
-    if (norm_b == 0.0) {
-        FG_CUDA(cudaMemsetAsync(d_x, 0, n * 8, s_));
-        FG_CUDA(cudaStreamSynchronize(s_));
-        if (st) *st = out;
-        return;
+    if (opt_.graph && !exec_) {
+        build_graph();
+        graph_tol_ = tol;
     }
-    // z = M^-1 r, p = z, rz = r.z
-    if (mixed) {
-        zf_ = enqueue_vcycle<float>(H32_, 0, r32_.p);
-        k_pcg_dots<float><<<row_blocks(n), TH, 0, s_>>>(n, r_.p, zf_, q_.p, 1, 1, partial_.p,
-                                                        sc_.p);
-        k_finish<<<1, FIN_TH, 0, s_>>>(partial_.p, row_blocks(n), FinDots{sc_.p, 1, 1});
-        k_pcg_p<float><<<row_blocks(n), TH, 0, s_>>>(n, zf_, p_.p, sc_.p, 1);
-    } else {
-        zd_ = enqueue_vcycle<double>(H64_, 0, r_.p);
-        k_pcg_dots<double><<<row_blocks(n), TH, 0, s_>>>(n, r_.p, zd_, q_.p, 0, 1, partial_.p,
-                                                         sc_.p);
-        k_finish<<<1, FIN_TH, 0, s_>>>(partial_.p, row_blocks(n), FinDots{sc_.p, 0, 1});
-        k_pcg_p<double><<<row_blocks(n), TH, 0, s_>>>(n, zd_, p_.p, sc_.p, 1);
-    }
-    FG_CHECK_LAUNCH();
-    if (opt_.graph && !exec_) build_loop_graph();
+    // The graph's stopping test keeps the tolerance of the solve that captured it.
+    if (exec_) h_init_->tol = graph_tol_;
     int status = FEMGPU_OK;
     std::string message;
-    double residual = std::sqrt(h_sc_->rr) / norm_b;
+    double residual = 0.0;
     size_t it = 0;
-    int restarts = 0;
-    for (;;) {
+    for (int restarts = 0;;) {
+        h_init_->iters = (int)std::min<size_t>(it, 0x7fffffff);
+        if (exec_)
+            run_graph(cancel);
+        else
+            run_launches(cancel);
+        const double norm_b = h_sc_->norm_b;
+        if (norm_b == 0.0) {
+            FG_CUDA(cudaMemsetAsync(d_x, 0, n * 8, s_));
+            FG_CUDA(cudaStreamSynchronize(s_));
+            if (st) *st = out;
+            return;
+        }
+        it = (size_t)h_sc_->iters;
+        residual = std::sqrt(h_sc_->rr) / norm_b;
+        if (h_sc_->bulk_timeout) break;  // reported below, before any other outcome
+        if (!(residual == residual)) {
+            status = FEMGPU_ERR_NOT_CONVERGED;
+            message = "conjugate gradients broke down: the residual is not a number";
+            break;
+        }
         // multigrid.rs:721-738: the residual test, then the iteration limit, then the cancel.
         if (residual <= tol) {
             // The true residual in FP64; with an FP32 preconditioner the recurrence can drift
             // from it, and then the solve restarts from x (iterative refinement).
-            k_pcg_residual<<<row_blocks(A64_.nslices * A64_.C), TH, 0, s_>>>(
-                SellOp<double>{A64_.view()}, b_.p, x_.p, t_.p, nullptr, partial_.p);
-            k_finish<<<1, FIN_TH, 0, s_>>>(partial_.p, row_blocks(A64_.nslices * A64_.C),
-                                       FinResidual0{sc_.p});
-            FG_CHECK_LAUNCH();
-            launches_ += 2;
-            FG_CUDA(cudaMemcpyAsync(h_sc_, sc_.p, sizeof(Scalars), cudaMemcpyDeviceToHost, s_));
-            FG_CUDA(cudaStreamSynchronize(s_));
-            double truth = std::sqrt(h_sc_->rr) / norm_b;
+            const double truth = std::sqrt(h_sc_->truth) / norm_b;
             out.true_residual = truth;
             if (truth <= tol || !mixed || restarts >= 3 || it >= max_iter) break;
             ++restarts;
-            FG_CUDA(cudaMemsetAsync(&sc_.p->done, 0, sizeof(int), s_));
-            k_pcg_residual<<<row_blocks(A64_.nslices * A64_.C), TH, 0, s_>>>(
-                SellOp<double>{A64_.view()}, b_.p, x_.p, r_.p, r32_.p, partial_.p);
-            k_finish<<<1, FIN_TH, 0, s_>>>(partial_.p, row_blocks(A64_.nslices * A64_.C),
-                                       FinResidual0{sc_.p});
-            zf_ = enqueue_vcycle<float>(H32_, 0, r32_.p);
-            k_pcg_dots<float><<<row_blocks(n), TH, 0, s_>>>(n, r_.p, zf_, q_.p, 1, 1, partial_.p,
-                                                            sc_.p);
-            k_finish<<<1, FIN_TH, 0, s_>>>(partial_.p, row_blocks(n), FinDots{sc_.p, 1, 1});
-            k_pcg_p<float><<<row_blocks(n), TH, 0, s_>>>(n, zf_, p_.p, sc_.p, 1);
-            FG_CHECK_LAUNCH();
-            launches_ += 5;
-            residual = truth;
             continue;
         }
-        if (it == max_iter) {
+        if (it >= max_iter) {
             char buf[200];
             std::snprintf(buf, sizeof buf,
                           "conjugate gradients did not converge: the residual is %s after %zu "
@@ -3270,22 +3430,6 @@ void SolverImpl::solve(const double* d_b, double* d_x, const volatile int* cance
         if (cancel && *cancel) {
             status = FEMGPU_ERR_CANCELLED;
             message = "cancelled";
-            break;
-        }
-        if (exec_) {
-            run_device_loop(cancel);
-            it = (size_t)h_sc_->iters;
-        } else {
-            enqueue_iteration();
-            FG_CUDA(cudaMemcpyAsync(h_sc_, sc_.p, sizeof(Scalars), cudaMemcpyDeviceToHost, s_));
-            FG_CUDA(cudaStreamSynchronize(s_));
-            ++it;
-        }
-        residual = std::sqrt(h_sc_->rr) / norm_b;
-        if (h_sc_->bulk_timeout) break;  // reported below, before any other outcome
-        if (!(residual == residual)) {
-            status = FEMGPU_ERR_NOT_CONVERGED;
-            message = "conjugate gradients broke down: the residual is not a number";
             break;
         }
     }
@@ -3338,9 +3482,8 @@ std::string SolverImpl::breakdown() {
     init.rz = 1.0;
     init.norm_b = 1.0;
     init.max_iter = 1;
+    init.tol = -1.0;
     FG_CUDA(cudaMemcpyAsync(sc_.p, &init, sizeof(Scalars), cudaMemcpyHostToDevice, s_));
-    double saved = tol;
-    tol = -1.0;
     std::vector<std::pair<std::string, cudaEvent_t>> trace;
     std::string out;
     for (int pass = 0; pass < 3; ++pass) {  // the last of 3 warm passes is reported
@@ -3352,7 +3495,6 @@ std::string SolverImpl::breakdown() {
         trace_ = nullptr;
         FG_CUDA(cudaStreamSynchronize(s_));
     }
-    tol = saved;
     double total = 0;
     char buf[200];
     for (size_t k = 1; k < trace.size(); ++k) {
@@ -3420,10 +3562,10 @@ void SolverImpl::kernel_time(int which, int reps, double* ms, double* bytes) {
             enqueue_spmv_pq();
         } else if (mixed) {
             MgLevel<float>& L = other ? S32 : H32_.levels.at(0);
-            enqueue_step(L, L.b.p, L.xa.p, 0.5f, 0.5f, L.xb.p);
+            enqueue_step(L, L.b.p, L.xa.p, 0.5f, 0.5f, L.d.p, L.d.p, L.xb.p);
         } else {
             MgLevel<double>& L = other ? S64 : H64_.levels.at(0);
-            enqueue_step(L, L.b.p, L.xa.p, 0.5, 0.5, L.xb.p);
+            enqueue_step(L, L.b.p, L.xa.p, 0.5, 0.5, L.d.p, L.d.p, L.xb.p);
         }
     };
     if (which == 0 && (mixed ? H32_.levels.empty() : H64_.levels.empty()))

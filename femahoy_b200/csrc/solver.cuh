@@ -118,6 +118,8 @@ void chebyshev(double lam, int degree, double lower, std::vector<double>* c1,
 struct Scalars {
     double bb, rr, rz, pq, alpha, beta, zq, norm_b;
     int done, iters, status, max_iter;
+    double tol;    // the relative residual of the stopping test
+    double truth;  // |b - A x|^2 at the end
     int bulk_timeout;  // a bulk-copy wait of the stencil tile kernels ran out of its limit
 };
 
@@ -285,19 +287,30 @@ class SolverImpl {
     template <class T>
     void build_levels(const std::vector<const DevCsr*>& mats, std::vector<DevRect>& ps,
                       const HostLevel& coarsest, Hierarchy<T>* H);
+    // The dot products that a cycle's last smoothing step takes along (q null: r.z alone).
+    struct Dots {
+        const double* q;
+    };
+    // `started`: the level's first smoothing step was done by the kernel before it (the finer
+    // level's restriction, or the update of r).
     template <class T>
-    // `started`: the level's first smoothing step was done by the finer level's restriction.
-    const T* enqueue_vcycle(Hierarchy<T>& H, size_t l, const T* b, bool started = false);
+    const T* enqueue_vcycle(Hierarchy<T>& H, size_t l, const T* b, bool started = false,
+                            const Dots* dots = nullptr);
     template <class T>
-    void enqueue_step(MgLevel<T>& L, const T* b, const T* xin, T c1, T c2, T* xout);
+    void enqueue_step(MgLevel<T>& L, const T* b, const T* xin, T c1, T c2, const T* din, T* dout,
+                      T* xout, const Dots* dots = nullptr);
     template <class T>
     void enqueue_residual(MgLevel<T>& L, const T* b, const T* x);
+    template <class T>
+    void enqueue_cycle(Hierarchy<T>& H, const T* r, bool started, bool init);
+    void enqueue_start();
     void enqueue_iteration();
+    void enqueue_truth();
     void enqueue_spmv_pq();
-    void build_loop_graph();
-    // Runs PCG iterations on the device until convergence, max_iter, a NaN or a cancel.
-    void run_device_loop(const volatile int* cancel);
-    void run_init(const double* d_b);
+    void build_graph();
+    // Solve from x_ until convergence, max_iter, a NaN or a cancel.
+    void run_graph(const volatile int* cancel);
+    void run_launches(const volatile int* cancel);
     void dense_direct(const HostCsr& a);
     // The Chebyshev degree of every level (1, 2 or 3) by timed trial solves, per size class.
     void tune_degree();
@@ -321,12 +334,11 @@ class SolverImpl {
     std::unique_ptr<SparseFactor> sparse_;  // the direct method above DENSE_DIRECT unknowns
     DevBuf<double> x_, r_, p_, q_, b_, z64_, t_;
     DevBuf<float> r32_;
-    const double* zd_ = nullptr;  // where the V-cycle leaves z (FP64 form)
-    const float* zf_ = nullptr;   // (mixed form)
     DevBuf<double> partial_;
     DevBuf<unsigned> counter_;
     DevBuf<Scalars> sc_;
-    Scalars* h_sc_ = nullptr;
+    Scalars* h_sc_ = nullptr;    // pinned: the scalars of the last solve
+    Scalars* h_init_ = nullptr;  // pinned: what a solve starts from
     DevBuf<int> done_zero_;
     cudaGraph_t graph_ = nullptr;
     cudaGraphExec_t exec_ = nullptr;
@@ -345,7 +357,10 @@ class SolverImpl {
     // Seconds of each phase of the setup, in the order first met (reported by describe()).
     std::vector<std::pair<std::string, double>> setup_s_;
     size_t launches_ = 0;      // kernels enqueued by the current solve
-    size_t graph_kernels_ = 0; // kernels of 1 iteration graph
+    bool in_graph_ = false;    // while the solve's graph is captured
+    double graph_tol_ = 0;     // the tolerance the graph was captured for
+    // The kernels of the graph: its start and end, and 1 iteration.
+    size_t fixed_kernels_ = 0, loop_kernels_ = 0;
 };
 
 }  // namespace femgpu

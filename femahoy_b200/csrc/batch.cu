@@ -417,103 +417,161 @@ __global__ void k_bgather(int64_t rows, const int64_t* __restrict__ ptr,
 
 // The members whose deepest level this is: out = M in for each, M its inverse, stored in tiles
 // of DTH = 32 rows, each tile by column (the 32 entries of column j of the tile contiguous). A
-// block takes 1 tile; its DW warps split the columns j into DW contiguous ranges. A warp takes
-// its columns 32 at a time: lane q brings the R right-side values of column j + q into the
-// warp's shared buffer (the next 32 already loading into registers while this 32 is used), then
-// lane i (row i of the tile) adds M[i][j] times the buffered values, the loads of M 8 columns
-// ahead. The DW partial sums are added in warp order through shared memory.
+// block takes 2 tiles (64 rows) and goes through the columns DK at a time: M's columns and the
+// right sides' rows come into shared memory by asynchronous copies, DSTAGES - 1 steps ahead; the
+// DW warps split a step's columns, lane i adding rows i and i + 32 of each column times the R
+// right-side values (a broadcast). The DW partial sums are added in warp order at the end. M does
+// not depend on the kernel before, so its first steps are asked for before the wait for it.
+//
+// What bounds it: M is read once (HBM) for 2 R operations per entry. With 1 row per lane and M
+// read into registers 8 columns at a time, the loads in flight (24 warps of 1 KB per SM) carried
+// 1.6 TB/s and the right sides' shared memory reads took as long as the products: 120 and 115 us
+// for the 2 large levels of 256 cantilevers with 16 load cases.
 constexpr int DW = 8;
-
+constexpr int DSTAGES = 3;
+constexpr int DMINB = 3;
 template <class T, int R>
-struct DenseChunk {
-    static constexpr int V = R % 4 == 0 ? R / 4 : R;  // loads of a row: 4-vectors, or scalars
-    typename std::conditional<R % 4 == 0, typename Vec4<T>::type, T>::type v[V];
-    __device__ __forceinline__ void load(const T* __restrict__ row, bool ok) {
-#pragma unroll
-        for (int k = 0; k < V; ++k) {
-            if constexpr (R % 4 == 0) {
-                if (ok) {
-                    v[k] = load4(row + 4 * k);
-                } else {
-                    v[k].x = v[k].y = v[k].z = v[k].w = 0;
-                }
-            } else {
-                v[k] = ok ? __ldg(row + k) : (T)0;
-            }
-        }
-    }
-    __device__ __forceinline__ void store(T* dst) const {
-#pragma unroll
-        for (int k = 0; k < V; ++k) {
-            if constexpr (R % 4 == 0) {
-                dst[4 * k] = v[k].x;
-                dst[4 * k + 1] = v[k].y;
-                dst[4 * k + 2] = v[k].z;
-                dst[4 * k + 3] = v[k].w;
-            } else {
-                dst[k] = v[k];
-            }
-        }
-    }
+struct DenseStage {
+    static constexpr int K = 256 / sizeof(T);  // columns per step
+    static constexpr int M = 2 * K * DTH, B = K * R;
+    static constexpr size_t BYTES = (size_t)DSTAGES * (M + B) * sizeof(T);
+    static_assert(BYTES >= (size_t)DW * DTH * (R + 1) * sizeof(T), "the partial sums fit");
+    // The right sides are copied in pieces of a row, at most 16 bytes.
+    static constexpr int PIECE = R * sizeof(T) < 16 ? R * sizeof(T) : 16;
 };
 
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void* to, const void* from) {
+    const unsigned t = (unsigned)__cvta_generic_to_shared(to);
+    if constexpr (BYTES == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(t), "l"(from) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(t), "l"(from), "n"(BYTES)
+                     : "memory");
+}
+
+// acc += m v over R right sides: in FP32 2 at a time (fma.rn.f32x2, each half rounded as a single
+// fused multiply-add), which leaves the other half of the issue slots to the loads.
 template <class T, int R>
-__global__ void __launch_bounds__(32 * DW)
+struct DenseSum {
+    T a[R];
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int c = 0; c < R; ++c) a[c] = 0;
+    }
+    __device__ __forceinline__ void add(T m, const T* __restrict__ v) {
+#pragma unroll
+        for (int c = 0; c < R; ++c) a[c] += m * v[c];
+    }
+    __device__ __forceinline__ T get(int c) const { return a[c]; }
+};
+template <int R>
+struct DenseSum2 {
+    unsigned long long a[R / 2];
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int c = 0; c < R / 2; ++c) a[c] = 0;
+    }
+    __device__ __forceinline__ void add(float m, const float* __restrict__ v) {
+        const unsigned b = __float_as_uint(m);
+        const unsigned long long mm = ((unsigned long long)b << 32) | b;
+        const ulonglong2* vv = reinterpret_cast<const ulonglong2*>(v);
+#pragma unroll
+        for (int c = 0; c < R / 4; ++c) {
+            const ulonglong2 x = vv[c];
+            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(a[2 * c]) : "l"(mm), "l"(x.x));
+            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(a[2 * c + 1]) : "l"(mm), "l"(x.y));
+        }
+    }
+    __device__ __forceinline__ float get(int c) const {
+        return __uint_as_float((unsigned)(c & 1 ? a[c / 2] >> 32 : a[c / 2]));
+    }
+};
+template <>
+struct DenseSum<float, 16> : DenseSum2<16> {};
+template <>
+struct DenseSum<float, 4> : DenseSum2<4> {};
+
+template <class T, int R>
+__global__ void __launch_bounds__(32 * DW, DMINB)
     k_bdense(const int2* __restrict__ tiles, const int64_t* __restrict__ off,
-             const int64_t* __restrict__ ioff, const T* __restrict__ inv,
-             const T* __restrict__ in, T* __restrict__ out) {
-    pdl_wait();
-    // Per warp a buffer of 32 right-side rows; reused at the end for the partial sums.
-    constexpr int STAGE = DW * 32 * R, PART = DW * DTH * (R + 1);
-    __shared__ T smem[STAGE > PART ? STAGE : PART];
+             const int64_t* __restrict__ ioff, const T* __restrict__ inv, const T* in,
+             T* __restrict__ out) {
+    typedef DenseStage<T, R> S;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T* smem = reinterpret_cast<T*>(smem_raw);
     const int2 tl = tiles[blockIdx.x];
-    const int64_t r0 = off[tl.x], m = off[tl.x + 1] - r0;
+    const int64_t r0 = off[tl.x];
+    const int m = (int)(off[tl.x + 1] - r0);
     const T* __restrict__ Mt = inv + ioff[tl.x] + (int64_t)tl.y * m;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const bool row_ok = tl.y + lane < m;
-    const int64_t j0 = m * w / DW, j1 = m * (w + 1) / DW;
-    T* buf = smem + w * 32 * R;
-    T acc[R];
+    const int halves = tl.y + DTH < m ? 2 : 1;
+    const int steps = (m + S::K - 1) / S::K;
+    auto fetch_m = [&](int t) {
+        if (t >= steps) return;
+        T* to = smem + (t % DSTAGES) * (S::M + S::B);
+        const int pieces = min(S::K, m - t * S::K) * DTH * (int)sizeof(T) / 16;
+        for (int h = 0; h < halves; ++h) {
+            const unsigned char* from = reinterpret_cast<const unsigned char*>(
+                Mt + (int64_t)h * DTH * m + (int64_t)t * S::K * DTH);
+            unsigned char* dst = reinterpret_cast<unsigned char*>(to + h * S::K * DTH);
+            for (int e = threadIdx.x; e < pieces; e += 32 * DW)
+                copy_async<16>(dst + 16 * e, from + 16 * e);
+        }
+    };
+    auto fetch_b = [&](int t) {
+        if (t < steps) {
+            unsigned char* dst =
+                reinterpret_cast<unsigned char*>(smem + (t % DSTAGES) * (S::M + S::B) + S::M);
+            const unsigned char* from =
+                reinterpret_cast<const unsigned char*>(in + (r0 + t * S::K) * R);
+            const int pieces = min(S::K, m - t * S::K) * R * (int)sizeof(T) / S::PIECE;
+            for (int e = threadIdx.x; e < pieces; e += 32 * DW)
+                copy_async<S::PIECE>(dst + S::PIECE * e, from + S::PIECE * e);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
 #pragma unroll
-    for (int c = 0; c < R; ++c) acc[c] = 0;
-    DenseChunk<T, R> next;
-    next.load(in + (r0 + j0 + lane) * R, j0 + lane < j1);
-    for (int64_t jc = j0; jc < j1; jc += 32) {
-        __syncwarp();
-        next.store(buf + lane * R);
-        __syncwarp();
-        if (jc + 32 < j1) next.load(in + (r0 + jc + 32 + lane) * R, jc + 32 + lane < j1);
-        const int nj = (int)min((int64_t)32, j1 - jc);
-        if (row_ok) {
-            int q = 0;
-            for (; q + 8 <= nj; q += 8) {
-                T mv[8];
+    for (int t = 0; t < DSTAGES - 1; ++t) fetch_m(t);
+    pdl_wait();
 #pragma unroll
-                for (int u = 0; u < 8; ++u) mv[u] = __ldg(Mt + 32 * (jc + q + u) + lane);
+    for (int t = 0; t < DSTAGES - 1; ++t) fetch_b(t);
+    DenseSum<T, R> acc0, acc1;
+    acc0.zero();
+    acc1.zero();
+    for (int t = 0; t < steps; ++t) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(DSTAGES - 2) : "memory");
+        __syncthreads();
+        fetch_m(t + DSTAGES - 1);
+        fetch_b(t + DSTAGES - 1);
+        const T* ms = smem + (t % DSTAGES) * (S::M + S::B) + lane;
+        const T* bs = smem + (t % DSTAGES) * (S::M + S::B) + S::M;
+        const int nj = min(S::K, m - t * S::K);
 #pragma unroll
-                for (int u = 0; u < 8; ++u)
-#pragma unroll
-                    for (int c = 0; c < R; ++c) acc[c] += mv[u] * buf[(q + u) * R + c];
-            }
-            for (; q < nj; ++q) {
-                const T mv = __ldg(Mt + 32 * (jc + q) + lane);
-#pragma unroll
-                for (int c = 0; c < R; ++c) acc[c] += mv * buf[q * R + c];
+        for (int u = 0; u < S::K / DW; ++u) {
+            const int k = w * (S::K / DW) + u;
+            if (k < nj) {
+                acc0.add(ms[k * DTH], bs + k * R);
+                acc1.add(ms[(S::K + k) * DTH], bs + k * R);
             }
         }
     }
-    __syncthreads();
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     T* part = smem;  // [DW][DTH][R + 1]
+    for (int h = 0; h < halves; ++h) {
+        __syncthreads();
 #pragma unroll
-    for (int c = 0; c < R; ++c) part[(w * DTH + lane) * (R + 1) + c] = acc[c];
-    __syncthreads();
-    for (int t = threadIdx.x; t < DTH * R; t += 32 * DW) {
-        const int row = t / R, c = t % R;
-        if (tl.y + row < m) {
-            T sum = 0;
+        for (int c = 0; c < R; ++c)
+            part[(w * DTH + lane) * (R + 1) + c] = h ? acc1.get(c) : acc0.get(c);
+        __syncthreads();
+        for (int t = threadIdx.x; t < DTH * R; t += 32 * DW) {
+            const int row = t / R, c = t % R, g = tl.y + h * DTH + row;
+            if (g < m) {
+                T sum = 0;
 #pragma unroll
-            for (int q = 0; q < DW; ++q) sum += part[(q * DTH + row) * (R + 1) + c];
-            out[(r0 + tl.y + row) * R + c] = sum;
+                for (int q = 0; q < DW; ++q) sum += part[(q * DTH + row) * (R + 1) + c];
+                out[(r0 + g) * R + c] = sum;
+            }
         }
     }
 }
@@ -1107,7 +1165,7 @@ struct BatchLevel {
     double lambda = 0;
     int ndense = 0, ntiles = 0;
     DevBuf<int64_t> doff, dioff;     // ndense + 1: first row (in the level), first inverse entry
-    DevBuf<int2> tiles;              // (dense member, first row of the tile)
+    DevBuf<int2> tiles;              // (dense member, first row of a pair of tiles)
     DevBuf<T> inv;
 };
 
@@ -1629,8 +1687,12 @@ void BatchImpl::build_levels(std::vector<SystemHierarchy>& H, std::vector<BatchL
                 off[j + 1] = off[j] + m;
                 // Row tiles of DTH rows (the last padded with zero rows), each stored by column.
                 ioff[j + 1] = ioff[j] + (m + DTH - 1) / DTH * DTH * m;
-                for (int64_t t = 0; t < m; t += DTH) tiles.push_back({j, (int)t});
+                for (int64_t t = 0; t < m; t += 2 * DTH) tiles.push_back({j, (int)t});
             }
+            // The longest rows first, so that the last blocks to start are short ones.
+            std::stable_sort(tiles.begin(), tiles.end(), [&](const int2& p, const int2& q) {
+                return off[p.x + 1] - off[p.x] > off[q.x + 1] - off[q.x];
+            });
             L.ntiles = (int)tiles.size();
             L.inv.alloc(ioff[L.ndense]);
             L.inv.zero(s_);  // the padding rows of each member's last tile
@@ -1728,7 +1790,10 @@ const T* BatchImpl::vcycle(std::vector<BatchLevel<T>>& Ls, size_t l, const T* b)
         launches_ += deg + 1;
     }
     if (L.ndense > 0) {
-        launch(true, k_bdense<T, R>, L.ntiles, 32 * DW, s_, L.tiles.p, L.doff.p, L.dioff.p,
+        constexpr size_t smem = DenseStage<T, R>::BYTES;
+        FG_CUDA(cudaFuncSetAttribute(k_bdense<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)smem));
+        launch_smem(true, k_bdense<T, R>, L.ntiles, 32 * DW, smem, s_, L.tiles.p, L.doff.p, L.dioff.p,
                L.inv.p, b, xa);
         FG_CHECK_LAUNCH();
         launches_ += 1;

@@ -140,12 +140,11 @@ __device__ __forceinline__ int64_t elem_of_thread() {
 // The first Chebyshev step from x = 0: d = c1 D^-1 b, x = d.
 template <class T, int R>
 __global__ void k_bcheb_first(int64_t n, const T* __restrict__ b, const T* __restrict__ dinv,
-                              T c1, T* __restrict__ d, T* __restrict__ x) {
+                              T c1, T* __restrict__ x) {
     pdl_wait();
     const int64_t t = elem_of_thread();
     if (t >= n * R) return;
     T v = c1 * dinv[t / R] * b[t];
-    d[t] = v;
     x[t] = v;
 }
 
@@ -182,21 +181,23 @@ __device__ __forceinline__ void sell_row_lanes(const SellView<T>& A, int row, in
     }
 }
 
-// d = c2 d + c1 D^-1 (b - A x), x_out = x + d.
+// d = c2 d + c1 D^-1 (b - A x), x_out = x + d. `din` null: c2 = 0 (the first step of a sweep);
+// `dout` null: no step reads this one's d.
 template <class T, int R>
 __global__ void __launch_bounds__(BTH)
     k_bcheb_step(SellView<T> A, const T* __restrict__ b, const T* __restrict__ xin,
-                 const T* __restrict__ dinv, T c1, T c2, T* __restrict__ d, T* __restrict__ xout) {
+                 const T* __restrict__ dinv, T c1, T c2, const T* din, T* dout,
+                 T* __restrict__ xout) {
     constexpr int W = Lanes<T, R>::W, P = R / W;
     pdl_wait();
     const int64_t t = elem_of_thread();
     if (t >= A.n * P) return;
     const int row = (int)(t / P), col = (int)(t % P) * W;
-    T acc[W], bb[W], dd[W], xx[W];
+    T acc[W], bb[W], dd[W] = {}, xx[W];
     sell_row_lanes<T, R>(A, row, col, xin, acc);
     const int64_t i = (int64_t)row * R + col;
     read_lanes<T, W>(b + i, bb);
-    read_lanes<T, W>(d + i, dd);
+    if (din) read_lanes<T, W>(din + i, dd);
     read_lanes<T, W>(xin + i, xx);
     const T di = dinv[row];
 #pragma unroll
@@ -205,7 +206,7 @@ __global__ void __launch_bounds__(BTH)
         dd[q] = c2 * dd[q] + c1 * di * r;
         xx[q] = xx[q] + dd[q];
     }
-    write_lanes<T, W>(d + i, dd);
+    if (dout) write_lanes<T, W>(dout + i, dd);
     write_lanes<T, W>(xout + i, xx);
 }
 
@@ -231,7 +232,9 @@ __global__ void __launch_bounds__(BTH)
 // the R / W threads of a block row takes W adjacent right sides, so that a block's column and 9
 // values are loaded once per W right sides and each x block row arrives as 16-byte vectors. Each
 // (row, right side) sum runs over the blocks in order, 3 terms per block, as with 1 right side
-// per thread.
+// per thread. B3_AHEAD blocks are summed at a time, the next ones' columns and values on their
+// way meanwhile.
+constexpr int B3_AHEAD = 1;
 template <class T, int R>
 __device__ __forceinline__ void bsell3_rows(const BSell3View<T>& A, int br, int col,
                                             const T* __restrict__ x,
@@ -240,105 +243,46 @@ __device__ __forceinline__ void bsell3_rows(const BSell3View<T>& A, int br, int 
     const int s = br / B3C, r = br % B3C;
     const int64_t b = A.slice_ptr[s], e = A.slice_ptr[s + 1];
     const int w = (int)((e - b) / B3C);
+    struct Batch {
+        uint32_t col[B3_AHEAD];
+        T v[B3_AHEAD][9];
+    };
+    auto load = [&](int k, Batch& o) {
+#pragma unroll
+        for (int u = 0; u < B3_AHEAD; ++u) {
+            const bool in = k + u < w;
+            const int64_t at = b + (int64_t)(k + u) * B3C;
+            o.col[u] = in ? __ldg(A.col + at + r) : (uint32_t)br;
+#pragma unroll
+            for (int q = 0; q < 9; ++q) o.v[u][q] = in ? __ldg(A.val + at * 9 + q * B3C + r) : (T)0;
+        }
+    };
 #pragma unroll
     for (int a = 0; a < 3; ++a)
 #pragma unroll
         for (int q = 0; q < W; ++q) acc[a][q] = 0;
-    // 2 blocks per pass: both columns, then both blocks' x rows and values in flight before
-    // the sums, which stay in block order.
-    int k = 0;
-    for (; k + 1 < w; k += 2) {
-        const int64_t blk = b + (int64_t)k * B3C + r;
-        const uint32_t J0 = __ldg(A.col + blk), J1 = __ldg(A.col + blk + B3C);
-        T xv[2][3][W], v[2][9];
+    Batch cur;
+    load(0, cur);
+    for (int k = 0; k < w; k += B3_AHEAD) {
+        T xv[B3_AHEAD][3][W];
 #pragma unroll
-        for (int h = 0; h < 3; ++h) {
-            load_lanes<T, W>(x + ((size_t)3 * J0 + h) * R + col, xv[0][h]);
-            load_lanes<T, W>(x + ((size_t)3 * J1 + h) * R + col, xv[1][h]);
-        }
+        for (int u = 0; u < B3_AHEAD; ++u)
 #pragma unroll
-        for (int e = 0; e < 9; ++e) {
-            v[0][e] = __ldg(A.val + blk * 9 + e);
-            v[1][e] = __ldg(A.val + (blk + B3C) * 9 + e);
-        }
+            for (int h = 0; h < 3; ++h)
+                load_lanes<T, W>(x + ((size_t)3 * cur.col[u] + h) * R + col, xv[u][h]);
+        Batch next;
+        load(k + B3_AHEAD, next);
 #pragma unroll
-        for (int u = 0; u < 2; ++u)
+        for (int u = 0; u < B3_AHEAD; ++u)
 #pragma unroll
             for (int a = 0; a < 3; ++a)
 #pragma unroll
                 for (int q = 0; q < W; ++q) {
-                    acc[a][q] += v[u][3 * a] * xv[u][0][q];
-                    acc[a][q] += v[u][3 * a + 1] * xv[u][1][q];
-                    acc[a][q] += v[u][3 * a + 2] * xv[u][2][q];
+                    acc[a][q] += cur.v[u][3 * a] * xv[u][0][q];
+                    acc[a][q] += cur.v[u][3 * a + 1] * xv[u][1][q];
+                    acc[a][q] += cur.v[u][3 * a + 2] * xv[u][2][q];
                 }
-    }
-    if (k < w) {
-        const int64_t blk = b + (int64_t)k * B3C + r;
-        const uint32_t J = __ldg(A.col + blk);
-        const T* v = A.val + blk * 9;
-        T x0[W], x1[W], x2[W];
-        load_lanes<T, W>(x + ((size_t)3 * J) * R + col, x0);
-        load_lanes<T, W>(x + ((size_t)3 * J + 1) * R + col, x1);
-        load_lanes<T, W>(x + ((size_t)3 * J + 2) * R + col, x2);
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            const T v0 = __ldg(v + 3 * a), v1 = __ldg(v + 3 * a + 1), v2 = __ldg(v + 3 * a + 2);
-#pragma unroll
-            for (int q = 0; q < W; ++q) {
-                acc[a][q] += v0 * x0[q];
-                acc[a][q] += v1 * x1[q];
-                acc[a][q] += v2 * x2[q];
-            }
-        }
-    }
-}
-
-// The sums of bsell3_rows for 1 right side `col` (the FP64 outer iteration's kernels, whose
-// dot products are formed per right side).
-template <class T, int R>
-__device__ __forceinline__ void bsell3_rows_col(const BSell3View<T>& A, int br, int col,
-                                                const T* __restrict__ x, T* acc) {
-    const int s = br / B3C, r = br % B3C;
-    const int64_t b = A.slice_ptr[s], e = A.slice_ptr[s + 1];
-    const int w = (int)((e - b) / B3C);
-    acc[0] = acc[1] = acc[2] = 0;
-    int k = 0;
-    for (; k + 1 < w; k += 2) {  // 2 blocks' loads in flight, the sums in block order
-        const int64_t blk = b + (int64_t)k * B3C + r;
-        const uint32_t J0 = __ldg(A.col + blk), J1 = __ldg(A.col + blk + B3C);
-        T xv[2][3], v[2][9];
-#pragma unroll
-        for (int h = 0; h < 3; ++h) {
-            xv[0][h] = __ldg(x + ((size_t)3 * J0 + h) * R + col);
-            xv[1][h] = __ldg(x + ((size_t)3 * J1 + h) * R + col);
-        }
-#pragma unroll
-        for (int e = 0; e < 9; ++e) {
-            v[0][e] = __ldg(A.val + blk * 9 + e);
-            v[1][e] = __ldg(A.val + (blk + B3C) * 9 + e);
-        }
-#pragma unroll
-        for (int u = 0; u < 2; ++u)
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                acc[a] += v[u][3 * a] * xv[u][0];
-                acc[a] += v[u][3 * a + 1] * xv[u][1];
-                acc[a] += v[u][3 * a + 2] * xv[u][2];
-            }
-    }
-    if (k < w) {
-        const int64_t blk = b + (int64_t)k * B3C + r;
-        const uint32_t J = __ldg(A.col + blk);
-        const T* v = A.val + blk * 9;
-        const T x0 = __ldg(x + ((size_t)3 * J) * R + col);
-        const T x1 = __ldg(x + ((size_t)3 * J + 1) * R + col);
-        const T x2 = __ldg(x + ((size_t)3 * J + 2) * R + col);
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            acc[a] += __ldg(v + 3 * a) * x0;
-            acc[a] += __ldg(v + 3 * a + 1) * x1;
-            acc[a] += __ldg(v + 3 * a + 2) * x2;
-        }
+        cur = next;
     }
 }
 
@@ -346,7 +290,7 @@ __device__ __forceinline__ void bsell3_rows_col(const BSell3View<T>& A, int br, 
 template <class T, int R>
 __global__ void __launch_bounds__(BTH)
     k_bcheb_step3(BSell3View<T> A, const T* __restrict__ b, const T* __restrict__ xin,
-                  const T* __restrict__ dinv, T c1, T c2, T* __restrict__ d,
+                  const T* __restrict__ dinv, T c1, T c2, const T* din, T* dout,
                   T* __restrict__ xout) {
     constexpr int W = Lanes<T, R>::W, P = R / W;
     pdl_wait();
@@ -358,9 +302,9 @@ __global__ void __launch_bounds__(BTH)
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         const int64_t row = 3 * (int64_t)br + a, i = row * R + col;
-        T bb[W], dd[W], xx[W];
+        T bb[W], dd[W] = {}, xx[W];
         read_lanes<T, W>(b + i, bb);
-        read_lanes<T, W>(d + i, dd);
+        if (din) read_lanes<T, W>(din + i, dd);
         read_lanes<T, W>(xin + i, xx);
         const T di = dinv[row];
 #pragma unroll
@@ -369,7 +313,7 @@ __global__ void __launch_bounds__(BTH)
             dd[q] = c2 * dd[q] + c1 * di * r;
             xx[q] = xx[q] + dd[q];
         }
-        write_lanes<T, W>(d + i, dd);
+        if (dout) write_lanes<T, W>(dout + i, dd);
         write_lanes<T, W>(xout + i, xx);
     }
 }
@@ -396,23 +340,55 @@ __global__ void __launch_bounds__(BTH)
     }
 }
 
-// out = M in (accumulate: out += M in) for a CSR transfer M, R columns.
+// out = M in (accumulate: out += M in) for a CSR transfer M, R columns: a thread takes 16 bytes of
+// adjacent columns of a row, GATHER_AHEAD entries' loads in flight at a time, each sum in the
+// row's order.
+constexpr int GATHER_AHEAD = 4;
 template <class T, int R>
-__global__ void k_bgather(int64_t rows, const int64_t* __restrict__ ptr,
-                          const uint32_t* __restrict__ idx, const T* __restrict__ val,
-                          const T* __restrict__ in, T* __restrict__ out, int accumulate) {
-    pdl_wait();
+__global__ void __launch_bounds__(BTH)
+    k_bgather(int64_t rows, const int64_t* __restrict__ ptr, const uint32_t* __restrict__ idx,
+              const T* __restrict__ val, const T* __restrict__ in, T* __restrict__ out,
+              int accumulate) {
+    constexpr int W = Lanes<T, R>::W, P = R / W;
     const int64_t t = elem_of_thread();
-    if (t >= rows * R) return;
-    const int64_t row = t / R;
-    const int col = (int)(t % R);
-    T s = 0;
-    for (int64_t k = ptr[row]; k < ptr[row + 1]; ++k)
-        s += val[k] * __ldg(in + (size_t)idx[k] * R + col);
-    if (accumulate)
-        out[t] += s;
-    else
-        out[t] = s;
+    const int64_t row = t / P;
+    const int col = (int)(t % P) * W;
+    int64_t e = 0, end = 0;
+    if (row < rows) {
+        e = __ldg(ptr + row);
+        end = __ldg(ptr + row + 1);
+    }
+    pdl_wait();
+    if (row >= rows) return;
+    T s[W];
+#pragma unroll
+    for (int q = 0; q < W; ++q) s[q] = 0;
+    for (; e < end; e += GATHER_AHEAD) {
+        uint32_t j[GATHER_AHEAD];
+        T v[GATHER_AHEAD], x[GATHER_AHEAD][W];
+#pragma unroll
+        for (int u = 0; u < GATHER_AHEAD; ++u) {
+            const int64_t k = e + u < end ? e + u : end - 1;
+            j[u] = __ldg(idx + k);
+            v[u] = __ldg(val + k);
+        }
+#pragma unroll
+        for (int u = 0; u < GATHER_AHEAD; ++u) load_lanes<T, W>(in + (size_t)j[u] * R + col, x[u]);
+#pragma unroll
+        for (int u = 0; u < GATHER_AHEAD; ++u)
+            if (e + u < end) {
+#pragma unroll
+                for (int q = 0; q < W; ++q) s[q] += v[u] * x[u][q];
+            }
+    }
+    const int64_t i = row * R + col;
+    if (accumulate) {
+        T o[W];
+        read_lanes<T, W>(out + i, o);
+#pragma unroll
+        for (int q = 0; q < W; ++q) s[q] = o[q] + s[q];
+    }
+    write_lanes<T, W>(out + i, s);
 }
 
 // The members whose deepest level this is: out = M in for each, M its inverse, stored in tiles
@@ -631,6 +607,28 @@ __device__ __forceinline__ void chunk_partial(double a, double b, double* __rest
     }
 }
 
+// The same for threads of W adjacent columns each.
+template <int R, int W>
+__device__ __forceinline__ void chunk_partial_lanes(const double (&a)[W], const double (&b)[W],
+                                                    double* __restrict__ partial) {
+    __shared__ double sa[BTH * W], sb[BTH * W];
+#pragma unroll
+    for (int q = 0; q < W; ++q) {
+        sa[threadIdx.x * W + q] = a[q];
+        sb[threadIdx.x * W + q] = b[q];
+    }
+    __syncthreads();
+    if (threadIdx.x < R) {
+        double ta = 0, tb = 0;
+        for (int k = threadIdx.x; k < BTH * W; k += R) {
+            ta += sa[k];
+            tb += sb[k];
+        }
+        partial[((int64_t)blockIdx.x * R + threadIdx.x) * 2] = ta;
+        partial[((int64_t)blockIdx.x * R + threadIdx.x) * 2 + 1] = tb;
+    }
+}
+
 // r = b - A x with the sums b.b and r.r (the exact FP64 operator); r and its FP32 copy are
 // written when their pointers are set.
 template <int R>
@@ -679,31 +677,40 @@ __global__ void __launch_bounds__(BTH)
 }
 
 // k_bpcg_residual and k_bpcg_spmv on the 3x3-block form of the exact operator: a chunk's rows
-// are whole nodes (multiples of 3), and a thread takes block rows of 1 column.
+// are whole nodes (multiples of 3), and a thread takes a block row's 16 bytes of adjacent columns
+// (with 1 column per thread, each block's column and values were loaded by twice the threads: the
+// FP64 residual of 256 cantilevers with 16 load cases took 172 us).
 template <int R>
 __global__ void __launch_bounds__(BTH)
     k_bpcg_residual3(BSell3View<double> A, const Chunk* __restrict__ chunks,
                      const double* __restrict__ b, const double* __restrict__ x,
                      double* __restrict__ r, float* __restrict__ r32,
                      double* __restrict__ partial) {
+    constexpr int W = Lanes<double, R>::W, P = R / W;
     pdl_wait();
     const Chunk ch = chunks[blockIdx.x];
-    const int col = threadIdx.x % R;
-    double bb = 0, rr = 0;
-    for (int br = ch.row0 / 3 + threadIdx.x / R; br < ch.row1 / 3; br += BTH / R) {
-        double acc[3];
-        bsell3_rows_col<double, R>(A, br, col, x, acc);
+    const int col = threadIdx.x % P * W;
+    double bb[W] = {}, rr[W] = {};
+    for (int br = ch.row0 / 3 + threadIdx.x / P; br < ch.row1 / 3; br += BTH / P) {
+        double acc[3][W];
+        bsell3_rows<double, R>(A, br, col, x, acc);
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
             const int64_t t = (3 * (int64_t)br + a) * R + col;
-            const double ri = b[t] - acc[a];
-            if (r) r[t] = ri;
-            if (r32) r32[t] = (float)ri;
-            bb += b[t] * b[t];
-            rr += ri * ri;
+            double bv[W];
+            read_lanes<double, W>(b + t, bv);
+#pragma unroll
+            for (int q = 0; q < W; ++q) {
+                const double ri = bv[q] - acc[a][q];
+                bb[q] += bv[q] * bv[q];
+                rr[q] += ri * ri;
+                acc[a][q] = ri;
+                if (r32) r32[t + q] = (float)ri;
+            }
+            if (r) write_lanes<double, W>(r + t, acc[a]);
         }
     }
-    chunk_partial<R>(bb, rr, partial);
+    chunk_partial_lanes<R, W>(bb, rr, partial);
 }
 
 template <int R>
@@ -712,24 +719,44 @@ __global__ void __launch_bounds__(BTH)
                  const double* __restrict__ p, double* __restrict__ q,
                  const int* __restrict__ done, double* __restrict__ partial,
                  const int* __restrict__ phase, const double* __restrict__ xv) {
+    constexpr int W = Lanes<double, R>::W, P = R / W;
     pdl_wait();
     const Chunk ch = chunks[blockIdx.x];
-    const int col = threadIdx.x % R;
+    const int col = threadIdx.x % P * W;
     const int seg = ch.sys * R + col;
-    const double* __restrict__ v = (phase && phase[seg] == PH_VERIFY) ? xv : p;
-    double pq = 0;
-    if (!done[seg])
-        for (int br = ch.row0 / 3 + threadIdx.x / R; br < ch.row1 / 3; br += BTH / R) {
-            double acc[3];
-            bsell3_rows_col<double, R>(A, br, col, v, acc);
+    // A streamed segment being verified takes q = A x (its true residual follows).
+    bool run[W], verify[W], any_p = false, any_x = false;
+#pragma unroll
+    for (int c = 0; c < W; ++c) {
+        run[c] = !done[seg + c];
+        verify[c] = phase && phase[seg + c] == PH_VERIFY;
+        any_p = any_p || (run[c] && !verify[c]);
+        any_x = any_x || (run[c] && verify[c]);
+    }
+    double pq[W] = {};
+    // The columns that take p, then those that take x; a thread's columns mostly agree.
+    for (int pass = 0; pass < 2; ++pass) {
+        if (!(pass ? any_x : any_p)) continue;
+        const double* __restrict__ v = pass ? xv : p;
+        for (int br = ch.row0 / 3 + threadIdx.x / P; br < ch.row1 / 3; br += BTH / P) {
+            double acc[3][W];
+            bsell3_rows<double, R>(A, br, col, v, acc);
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
                 const int64_t t = (3 * (int64_t)br + a) * R + col;
-                q[t] = acc[a];
-                pq += v[t] * acc[a];
+                double vv[W];
+                read_lanes<double, W>(v + t, vv);
+#pragma unroll
+                for (int c = 0; c < W; ++c)
+                    if (run[c] && verify[c] == (pass == 1)) {
+                        q[t + c] = acc[a][c];
+                        pq[c] += vv[c] * acc[a][c];
+                    }
             }
         }
-    chunk_partial<R>(pq, 0.0, partial);
+    }
+    const double zero[W] = {};
+    chunk_partial_lanes<R, W>(pq, zero, partial);
 }
 
 // x += alpha p, r -= alpha q (multigrid.rs:742-745) with the sums r.r.
@@ -1756,19 +1783,23 @@ const T* BatchImpl::vcycle(std::vector<BatchLevel<T>>& Ls, size_t l, const T* b)
     if (L.ns > 0) {
         const int g = (int)((L.ns * R + BTH - 1) / BTH);
         const int deg = (int)L.c1.size();
-        launch(true, k_bcheb_first<T, R>, g, BTH, s_, L.ns, b, L.dinv.p, (T)L.c1[0], L.d.p, xa);
+        launch(true, k_bcheb_first<T, R>, g, BTH, s_, L.ns, b, L.dinv.p, (T)L.c1[0], xa);
         const int g3 = (int)((L.ns / 3 * (R / Lanes<T, R>::W) + BTH - 1) / BTH);
         const int gs = (int)((L.ns * (R / Lanes<T, R>::W) + BTH - 1) / BTH);
-        auto step = [&](const T* xin, T* xout, int k) {
+        // After the first step d is x itself; the first step of the second sweep has c2 = 0, and no
+        // step reads the last one's d of a sweep.
+        auto step = [&](const T* xin, T* xout, int k, bool first_sweep) {
+            const T* din = k == 0 ? nullptr : k == 1 && first_sweep ? xin : (const T*)L.d.p;
+            T* dout = k + 1 < deg ? L.d.p : nullptr;
             if (L.block3)
                 launch(true, k_bcheb_step3<T, R>, g3, BTH, s_, L.view3(), b, xin, L.dinv.p,
-                       (T)L.c1[k], (T)L.c2[k], L.d.p, xout);
+                       (T)L.c1[k], (T)L.c2[k], din, dout, xout);
             else
                 launch(true, k_bcheb_step<T, R>, gs, BTH, s_, L.A.view(), b, xin, L.dinv.p,
-                       (T)L.c1[k], (T)L.c2[k], L.d.p, xout);
+                       (T)L.c1[k], (T)L.c2[k], din, dout, xout);
         };
         for (int k = 1; k < deg; ++k) {
-            step(xa, xb, k);
+            step(xa, xb, k, true);
             std::swap(xa, xb);
         }
         if (L.block3)
@@ -1776,14 +1807,14 @@ const T* BatchImpl::vcycle(std::vector<BatchLevel<T>>& Ls, size_t l, const T* b)
         else
             launch(true, k_bresidual<T, R>, gs, BTH, s_, L.A.view(), b, xa, L.r.p);
         T* bc = Ls[l + 1].b.p;
-        const int gc = (int)((L.nc * R + BTH - 1) / BTH);
+        const int gc = (int)((L.nc * (R / Lanes<T, R>::W) + BTH - 1) / BTH);
         launch(true, k_bgather<T, R>, gc, BTH, s_, L.nc, L.rptr.p, L.ridx.p, L.rval.p, L.r.p, bc, 0);
         FG_CHECK_LAUNCH();
         launches_ += deg + 2;
         const T* ec = vcycle<T, R>(Ls, l + 1, bc);
-        launch(true, k_bgather<T, R>, g, BTH, s_, L.ns, L.pptr.p, L.pidx.p, L.pval.p, ec, xa, 1);
+        launch(true, k_bgather<T, R>, gs, BTH, s_, L.ns, L.pptr.p, L.pidx.p, L.pval.p, ec, xa, 1);
         for (int k = 0; k < deg; ++k) {
-            step(xa, xb, k);
+            step(xa, xb, k, false);
             std::swap(xa, xb);
         }
         FG_CHECK_LAUNCH();
@@ -1793,8 +1824,8 @@ const T* BatchImpl::vcycle(std::vector<BatchLevel<T>>& Ls, size_t l, const T* b)
         constexpr size_t smem = DenseStage<T, R>::BYTES;
         FG_CUDA(cudaFuncSetAttribute(k_bdense<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem));
-        launch_smem(true, k_bdense<T, R>, L.ntiles, 32 * DW, smem, s_, L.tiles.p, L.doff.p, L.dioff.p,
-               L.inv.p, b, xa);
+        launch_smem(true, k_bdense<T, R>, L.ntiles, 32 * DW, smem, s_, L.tiles.p, L.doff.p,
+                    L.dioff.p, L.inv.p, b, xa);
         FG_CHECK_LAUNCH();
         launches_ += 1;
     }
@@ -2214,10 +2245,10 @@ void BatchImpl::kernel_time(int reps, double* ms, double* bytes) {
             if (k == 5) FG_CUDA(cudaEventRecord(ev0_, s_));
             if (L.block3)
                 k_bcheb_step3<T, R><<<g3, BTH, 0, s_>>>(L.view3(), L.b.p, L.xa.p, L.dinv.p,
-                                                         (T)0.5, (T)0.5, L.d.p, L.xb.p);
+                                                         (T)0.5, (T)0.5, L.d.p, L.d.p, L.xb.p);
             else
                 k_bcheb_step<T, R><<<g, BTH, 0, s_>>>(L.A.view(), L.b.p, L.xa.p, L.dinv.p,
-                                                      (T)0.5, (T)0.5, L.d.p, L.xb.p);
+                                                      (T)0.5, (T)0.5, L.d.p, L.d.p, L.xb.p);
         }
         FG_CHECK_LAUNCH();
         FG_CUDA(cudaEventRecord(ev1_, s_));

@@ -175,7 +175,7 @@ template <class T>
 __global__ void k_b3_fill(const int64_t* __restrict__ ptr, const uint32_t* __restrict__ idx,
                           const double* __restrict__ val, int64_t nb,
                           const int64_t* __restrict__ sptr, const uint32_t* __restrict__ row,
-                          uint32_t* __restrict__ col, T* __restrict__ vals, bool planes) {
+                          uint32_t* __restrict__ col, T* __restrict__ vals) {
     for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < nb;
          g += (int64_t)gridDim.x * blockDim.x) {
         const int64_t I = row ? (int64_t)row[g] : g;
@@ -188,8 +188,7 @@ __global__ void k_b3_fill(const int64_t* __restrict__ ptr, const uint32_t* __res
                 col[blk] = idx[ptr[3 * I] + 3 * k] / 3;
                 for (int q = 0; q < 3; ++q)
                     for (int c = 0; c < 3; ++c)
-                        vals[planes ? (blk - r) * 9 + (3 * q + c) * B3C + r
-                                    : blk * 9 + 3 * q + c] =
+                        vals[(blk - r) * 9 + (3 * q + c) * B3C + r] =
                             (T)val[ptr[3 * I + q] + 3 * k + c];
             } else {
                 col[blk] = (uint32_t)I;  // padding: value 0, the block row's own x
@@ -297,8 +296,7 @@ bool make_bsell3_device(const DevCsr& a, DevBuf<int64_t>* sptr, DevBuf<uint32_t>
     col->zero(s);
     val->zero(s);
     k_b3_fill<T><<<blocks_for(nb, TH), TH, 0, s>>>(a.ptr.p, a.idx.p, a.val.p, nb, sptr->p,
-                                                   row ? row->p : nullptr, col->p, val->p,
-                                                   row != nullptr);
+                                                   row ? row->p : nullptr, col->p, val->p);
     FG_CHECK_LAUNCH();
     return true;
 }

@@ -36,10 +36,9 @@ void fill_offsets(const int64_t* ptr, const uint32_t* idx, const double* val, in
                   T* coef, cudaStream_t s);
 
 // The 3x3-block SELL form of `a` (block3.cuh): false, and nothing built, unless every node's 3
-// rows have the same columns and the columns come in aligned triples. With `row`: the values
-// in the planes of Block3Op, the block rows of a window sorted by width where that stores fewer
-// blocks (`row` then gets the block row of each slot, else it stays empty). Without: each block's
-// 9 values together, the block rows in order.
+// rows have the same columns and the columns come in aligned triples. With `row`, the block rows of
+// a window are sorted by width where that stores fewer blocks (`row` then gets the block row of each
+// slot, else it stays empty).
 template <class T>
 bool make_bsell3_device(const DevCsr& a, DevBuf<int64_t>* sptr, DevBuf<uint32_t>* col,
                         DevBuf<T>* val, DevBuf<uint32_t>* row, cudaStream_t s);

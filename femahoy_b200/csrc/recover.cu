@@ -10,11 +10,21 @@
 // order) and, beside it, the place (0-9) of the point in each of those cells. A recovery first
 // copies u into 32 bytes per point, so that each point's displacement is 1 aligned 32-byte load.
 //
-// One thread per point walks its cells in increasing order, evaluates Tet10::strain_stress
-// (tet10.rs:142-169) at its own volume coordinates in each, and sums. The reference adds the same
-// terms to the same point in the same order, so the means are bit-identical with it. Each
-// (cell, point) pair, a "visit", is evaluated exactly once, by the thread of its point. The unit
-// is compiled with -fmad=false, so no multiply and add are fused.
+// A recovery evaluates Tet10::strain_stress (tet10.rs:142-169) at each (cell, point) pair, a
+// "visit", exactly once, and each point sums its visits in increasing cell order. The reference
+// adds the same terms to the same point in the same order, so the means are bit-identical with
+// it. The unit is compiled with -fmad=false, so no multiply and add are fused.
+//
+// The visits are evaluated cell by cell (a thread takes 10 or 2 of a cell, with its record, points
+// and displacements in registers), leaving strain, dt and material in 64 bytes each; then a thread
+// per point gathers its visits' 64 bytes and forms their stresses and the means. What bounds it:
+// the FP64 operations of the visits (about 300 each) and the visits' 64 bytes written and read.
+// With a thread per point evaluating its own visits, the lanes of a warp sat in different cells,
+// so each load of a record, a point number or a displacement touched up to 32 lines and the L1
+// set the time: 531 us for the 160 x 20 x 20 P2 beam (384,000 cells, 3.84M visits; the 3 largest
+// kernels by CUDA events 482), now 283 (180 for the visits, 96 for the means); 239 -> 51 us for
+// 15,360 cells, where each block also raised its parts' maxima from nothing.
+// That form serves meshes whose visits would take more than VISIT_BYTES_MAX.
 //
 // Peaks: the thread of each visit folds its von Mises stress into 3 running maxima of its part,
 // each a 128-bit word updated by compare-and-swap: (value, ~key) for the peak and for the
@@ -210,24 +220,8 @@ __global__ void k_pad_u(const double* __restrict__ u, int64_t npoints, double* _
     }
 }
 
-// Tet10::strain_stress (tet10.rs:142-169) of cell e (record rp, points t) at its point c,
-// followed by reorder and tensor_strain (elastic.rs:967-975): sig and eps in the order xx, yy,
-// zz, xy, yz, xz.
-__device__ __forceinline__ void strain_stress_l(const CellRecord* __restrict__ rp,
-                                                const MaterialEntry* __restrict__ mats,
-                                                const uint32_t t[10], const double l[4],
-                                                const double* __restrict__ u4,
-                                                const double* __restrict__ dtemp,
-                                                double sig[6], double eps[6], uint32_t* tag);
-
-__device__ __forceinline__ void strain_stress_at(const CellRecord* __restrict__ rp,
-                                                 const MaterialEntry* __restrict__ mats,
-                                                 const uint32_t t[10], int c,
-                                                 const double* __restrict__ u4,
-                                                 const double* __restrict__ dtemp,
-                                                 double sig[6], double eps[6], uint32_t* tag) {
-    // node_coordinates (tet10.rs:216-228)
-    double l[4];
+// node_coordinates (tet10.rs:216-228): the volume coordinates of place c of a cell.
+__device__ __forceinline__ void place_coordinates(int c, double l[4]) {
     if (c < 4) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) l[k] = k == c ? 1.0 : 0.0;
@@ -236,25 +230,40 @@ __device__ __forceinline__ void strain_stress_at(const CellRecord* __restrict__ 
 #pragma unroll
         for (int k = 0; k < 4; ++k) l[k] = (k == i || k == j) ? 0.5 : 0.0;
     }
-    strain_stress_l(rp, mats, t, l, u4, dtemp, sig, eps, tag);
 }
 
-// Tet10::strain_stress (tet10.rs:142-169) of cell e at the volume coordinates l, with reorder
-// and tensor_strain as above.
-__device__ __forceinline__ void strain_stress_l(const CellRecord* __restrict__ rp,
-                                                const MaterialEntry* __restrict__ mats,
-                                                const uint32_t t[10], const double l[4],
-                                                const double* __restrict__ u4,
-                                                const double* __restrict__ dtemp,
-                                                double sig[6], double eps[6], uint32_t* tag) {
+// What the strain of a cell needs: the gradients of its volume coordinates, its points'
+// displacements and its corners' temperature changes (0 without any).
+struct CellState {
+    double g[12], u[10][3], dtemp[4];
+    uint32_t mat, tag;
+};
+
+__device__ __forceinline__ void load_cell(const CellRecord* __restrict__ rp, const uint32_t t[10],
+                                          const double* __restrict__ u4,
+                                          const double* __restrict__ dtemp, CellState* s) {
     const double* rd = reinterpret_cast<const double*>(rp);
-    double g[12];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) ld32(rd + 4 * k, g[4 * k], g[4 * k + 1], g[4 * k + 2], g[4 * k + 3]);
+    for (int k = 0; k < 3; ++k)
+        ld32(rd + 4 * k, s->g[4 * k], s->g[4 * k + 1], s->g[4 * k + 2], s->g[4 * k + 3]);
     const uint2 mt = __ldg(reinterpret_cast<const uint2*>(rd + 12));
-    const uint32_t mat = mt.x;
-    *tag = mt.y;
-    double e[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    s->mat = mt.x;
+    s->tag = mt.y;
+    double unused;
+#pragma unroll
+    for (int i = 0; i < 10; ++i)
+        ld32(u4 + 4 * (int64_t)t[i], s->u[i][0], s->u[i][1], s->u[i][2], unused);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) s->dtemp[k] = dtemp ? __ldg(dtemp + t[k]) : 0.0;
+}
+
+// The strain of Tet10::strain_stress (tet10.rs:142-169) at the volume coordinates l, and the
+// temperature change there.
+__device__ __forceinline__ void strain_of(const CellState& s, const double l[4], double e[6],
+                                          double* dt_out) {
+    const double* g = s.g;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) e[i] = 0.0;
 #pragma unroll
     for (int i = 0; i < 10; ++i) {
         // The gradient of function i at l (tet10.rs:77-87).
@@ -268,8 +277,7 @@ __device__ __forceinline__ void strain_stress_l(const CellRecord* __restrict__ r
 #pragma unroll
             for (int d = 0; d < 3; ++d) gi[d] = 4.0 * (l[a] * g[3 * b + d] + l[b] * g[3 * a + d]);
         }
-        double ui[3], unused;
-        ld32(u4 + 4 * (int64_t)t[i], ui[0], ui[1], ui[2], unused);
+        const double* ui = s.u[i];
 #pragma unroll
         for (int a = 0; a < 3; ++a) e[a] += gi[a] * ui[a];
         // SHEAR (tet10.rs:41): yz, xz, xy
@@ -279,7 +287,15 @@ __device__ __forceinline__ void strain_stress_l(const CellRecord* __restrict__ r
     }
     double dt = -0.0;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) dt += l[k] * (dtemp ? __ldg(dtemp + t[k]) : 0.0);
+    for (int k = 0; k < 4; ++k) dt += l[k] * s.dtemp[k];
+    *dt_out = dt;
+}
+
+// The stress of the strain e (hex.rs:128-139), with reorder and tensor_strain
+// (elastic.rs:967-975): sig and eps in the order xx, yy, zz, xy, yz, xz.
+__device__ __forceinline__ void stress_of(const MaterialEntry* __restrict__ mats, uint32_t mat,
+                                          const double e[6], double dt, double sig[6],
+                                          double eps[6]) {
     const double* md = reinterpret_cast<const double*>(mats + mat);
     double w[16];
 #pragma unroll
@@ -287,7 +303,7 @@ __device__ __forceinline__ void strain_stress_l(const CellRecord* __restrict__ r
     // w[0..9) normal, w[9..12) shear, w[12..15) thermal.
     double s[6];
 #pragma unroll
-    for (int a = 0; a < 3; ++a)  // hex.rs:128-139
+    for (int a = 0; a < 3; ++a)
         s[a] = w[3 * a] * e[0] + w[3 * a + 1] * e[1] + w[3 * a + 2] * e[2];
 #pragma unroll
     for (int k = 0; k < 3; ++k) s[3 + k] = w[9 + k] * e[3 + k];
@@ -307,6 +323,32 @@ __device__ __forceinline__ void strain_stress_l(const CellRecord* __restrict__ r
     eps[5] = 0.5 * e[4];
 }
 
+// Both at the volume coordinates l, and at place c.
+__device__ __forceinline__ void strain_stress_l(const CellRecord* __restrict__ rp,
+                                                const MaterialEntry* __restrict__ mats,
+                                                const uint32_t t[10], const double l[4],
+                                                const double* __restrict__ u4,
+                                                const double* __restrict__ dtemp,
+                                                double sig[6], double eps[6], uint32_t* tag) {
+    CellState s;
+    load_cell(rp, t, u4, dtemp, &s);
+    *tag = s.tag;
+    double e[6], dt;
+    strain_of(s, l, e, &dt);
+    stress_of(mats, s.mat, e, dt, sig, eps);
+}
+
+__device__ __forceinline__ void strain_stress_at(const CellRecord* __restrict__ rp,
+                                                 const MaterialEntry* __restrict__ mats,
+                                                 const uint32_t t[10], int c,
+                                                 const double* __restrict__ u4,
+                                                 const double* __restrict__ dtemp,
+                                                 double sig[6], double eps[6], uint32_t* tag) {
+    double l[4];
+    place_coordinates(c, l);
+    strain_stress_l(rp, mats, t, l, u4, dtemp, sig, eps, tag);
+}
+
 // max(*a, v) by compare-and-swap. The high half of *a never decreases, so a v whose high half
 // is below it is below *a and needs no atomic.
 __device__ __forceinline__ void fold_max(u128* a, u128 v) {
@@ -319,6 +361,156 @@ __device__ __forceinline__ void fold_max(u128* a, u128 v) {
         const u128 prev = atomicCAS(a, old, v);
         if (prev == old) break;
         old = prev;  // another thread raised it: compare again
+    }
+}
+
+// The fold of 1 visit (cell e, place c) into the 3 maxima of its part.
+__device__ __forceinline__ void fold_visit(u128* fold, uint32_t e, int c, uint32_t tag, bool sing_v,
+                                           const double sig[6]) {
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(mises6(sig));
+    const unsigned long long key = 10ull * e + c;
+    const int p = (int)(tag & ~NEAR_BIT);
+    const bool reg = !(tag & NEAR_BIT) && !sing_v;
+    const bool nan = is_nan_bits(bits);
+    const u128 vk = ((u128)bits << 64) | (u128)(NONE - key);
+    if (!nan) fold_max(fold + 3 * p, vk);
+    if (reg) {
+        if (!nan) fold_max(fold + 3 * p + 1, vk);
+        fold_max(fold + 3 * p + 2, ((u128)(NONE - key) << 64) | (u128)bits);
+    }
+}
+
+// The means of elastic_tet.rs:419-425 from the sums of `count` visits, and elastic_tet.rs:482-483.
+__device__ __forceinline__ void write_point(int64_t v, int64_t count, double ss[6], double se[6],
+                                            double* __restrict__ stress,
+                                            double* __restrict__ strain,
+                                            double* __restrict__ mises_out,
+                                            double* __restrict__ principal_out) {
+    const double cnt = (double)(count > 1 ? count : 1);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        ss[i] /= cnt;
+        se[i] /= cnt;
+        stress[6 * v + i] = ss[i];
+        strain[6 * v + i] = se[i];
+    }
+    if (mises_out) mises_out[v] = mises6(ss);
+    if (principal_out) {
+        double pr[3];
+        principal3(ss, pr);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) principal_out[3 * v + i] = pr[i];
+    }
+}
+
+// The most that the visits' 64 bytes may take.
+constexpr size_t VISIT_BYTES_MAX = (size_t)4 << 30;
+// From this many cells on a thread takes all 10 visits of a cell.
+constexpr int64_t WHOLE_CELLS = 100'000;
+constexpr int VISIT_BLOCKS = 8;  // blocks per SM
+
+// A 32-byte store; p is 32-byte aligned.
+__device__ __forceinline__ void st32(double* p, double a, double b, double c, double d) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d)
+                 : "memory");
+}
+
+// A thread per N of a cell's 10 visits 10 e + c: the strain (6), dt and material number (as bits)
+// of each into 64 bytes, and with PEAKS the peaks of elastic_tet.rs:405-416 into `peak` (3 words per
+// part: peak, regular peak, first regular visit), through shared memory when SMEM. The blocks are
+// few and go on to further cells, so that most visits meet maxima that they do not raise.
+template <bool PEAKS, bool SMEM, int N>
+__global__ void __launch_bounds__(128)
+    k_visit_strains(const CellRecord* __restrict__ rec, const MaterialEntry* __restrict__ mats,
+                    const uint32_t* __restrict__ t10, const double* __restrict__ u4,
+                    const double* __restrict__ dtemp, const uint8_t* __restrict__ singular,
+                    int64_t nel, int nparts, double* __restrict__ visits,
+                    u128* __restrict__ peak) {
+    static_assert(10 % N == 0, "a thread's visits are of 1 cell");
+    extern __shared__ u128 peak_s[];
+    u128* fold = SMEM ? peak_s : peak;
+    if (PEAKS && SMEM) {
+        for (int i = threadIdx.x; i < 3 * nparts; i += blockDim.x) peak_s[i] = 0;
+        __syncthreads();
+    }
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < nel * (10 / N);
+         q += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t cell = (uint32_t)(q / (10 / N));
+        const int c0 = (int)(q - (int64_t)cell * (10 / N)) * N;
+        const uint2* row = reinterpret_cast<const uint2*>(t10 + 10 * (int64_t)cell);
+        uint32_t t[10];
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            const uint2 w = __ldg(row + k);
+            t[2 * k] = w.x;
+            t[2 * k + 1] = w.y;
+        }
+        CellState s;
+        load_cell(rec + cell, t, u4, dtemp, &s);
+#pragma unroll 1
+        for (int c = c0; c < c0 + N; ++c) {
+            const int64_t k = 10 * (int64_t)cell + c;
+            double l[4], e[6], dt;
+            place_coordinates(c, l);
+            strain_of(s, l, e, &dt);
+            st32(visits + 8 * k, e[0], e[1], e[2], e[3]);
+            st32(visits + 8 * k + 4, e[4], e[5], dt, __longlong_as_double((long long)s.mat));
+            if (PEAKS) {
+                double sig[6], eps[6];
+                stress_of(mats, s.mat, e, dt, sig, eps);
+                const bool sing_v = singular && singular[__ldg(t10 + k)];
+                fold_visit(fold, cell, c, s.tag, sing_v, sig);
+            }
+        }
+    }
+    if (PEAKS && SMEM) {
+        __syncthreads();
+        for (int i = threadIdx.x; i < 3 * nparts; i += blockDim.x)
+            if (peak_s[i] != 0) fold_max(peak + i, peak_s[i]);
+    }
+}
+
+// A thread per point: the sums of elastic_tet.rs:396-403 over its visits in increasing cell order.
+constexpr int MEANS_AHEAD = 3;
+__global__ void __launch_bounds__(128)
+    k_visit_means(const double* __restrict__ visits, const MaterialEntry* __restrict__ mats,
+                  const int64_t* __restrict__ start, const uint32_t* __restrict__ of_node,
+                  const uint8_t* __restrict__ place, int64_t npoints,
+                  double* __restrict__ stress, double* __restrict__ strain,
+                  double* __restrict__ mises_out, double* __restrict__ principal_out) {
+    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < npoints;
+         v += (int64_t)gridDim.x * blockDim.x) {
+        double ss[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        double se[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        const int64_t b = start[v], end = start[v + 1];
+        // MEANS_AHEAD visits' loads in flight, summed in order; past the end the last one's again.
+        for (int64_t k = b; k < end; k += MEANS_AHEAD) {
+            const double* at[MEANS_AHEAD];
+            double e[MEANS_AHEAD][6], dt[MEANS_AHEAD], bits[MEANS_AHEAD];
+#pragma unroll
+            for (int h = 0; h < MEANS_AHEAD; ++h) {
+                const int64_t j = k + h < end ? k + h : end - 1;
+                at[h] = visits + 8 * (10 * (int64_t)__ldg(of_node + j) + __ldg(place + j));
+            }
+#pragma unroll
+            for (int h = 0; h < MEANS_AHEAD; ++h) {
+                ld32(at[h], e[h][0], e[h][1], e[h][2], e[h][3]);
+                ld32(at[h] + 4, e[h][4], e[h][5], dt[h], bits[h]);
+            }
+#pragma unroll
+            for (int h = 0; h < MEANS_AHEAD; ++h)
+                if (k + h < end) {
+                    double sig[6], eps[6];
+                    stress_of(mats, (uint32_t)__double_as_longlong(bits[h]), e[h], dt[h], sig,
+                              eps);
+#pragma unroll
+                    for (int i = 0; i < 6; ++i) {
+                        ss[i] += sig[i];
+                        se[i] += eps[i];
+                    }
+                }
+        }
+        write_point(v, end - b, ss, se, stress, strain, mises_out, principal_out);
     }
 }
 
@@ -367,37 +559,9 @@ __global__ void __launch_bounds__(128, 4)
                 ss[i] += sig[i];
                 se[i] += eps[i];
             }
-            if (PEAKS) {
-                const unsigned long long bits =
-                    (unsigned long long)__double_as_longlong(mises6(sig));
-                const unsigned long long key = 10ull * e + c;
-                const int p = (int)(tg & ~NEAR_BIT);
-                const bool reg = !(tg & NEAR_BIT) && !sing_v;
-                const bool nan = is_nan_bits(bits);
-                const u128 vk = ((u128)bits << 64) | (u128)(NONE - key);
-                if (!nan) fold_max(fold + 3 * p, vk);
-                if (reg) {
-                    if (!nan) fold_max(fold + 3 * p + 1, vk);
-                    fold_max(fold + 3 * p + 2, ((u128)(NONE - key) << 64) | (u128)bits);
-                }
-            }
+            if (PEAKS) fold_visit(fold, e, c, tg, sing_v, sig);
         }
-        int64_t count = end - b;
-        const double cnt = (double)(count > 1 ? count : 1);
-#pragma unroll
-        for (int i = 0; i < 6; ++i) {
-            ss[i] /= cnt;
-            se[i] /= cnt;
-            stress[6 * v + i] = ss[i];
-            strain[6 * v + i] = se[i];
-        }
-        if (mises_out) mises_out[v] = mises6(ss);
-        if (principal_out) {
-            double pr[3];
-            principal3(ss, pr);
-#pragma unroll
-            for (int i = 0; i < 3; ++i) principal_out[3 * v + i] = pr[i];
-        }
+        write_point(v, end - b, ss, se, stress, strain, mises_out, principal_out);
     }
     if (PEAKS && SMEM) {
         __syncthreads();
@@ -809,6 +973,7 @@ struct femgpu_recovery {
     DevBuf<MaterialEntry> mats;
     DevBuf<uint8_t> singular;
     DevBuf<double> u4;
+    DevBuf<double> visits;  // 8 per visit; empty where they would take too much memory
     DevBuf<u128> peak;
     DevBuf<femgpu_peak> dpeaks;
     // Device copies for the host-pointer form.
@@ -820,6 +985,21 @@ struct femgpu_recovery {
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
         if (s) cudaStreamDestroy(s);
+    }
+
+    template <int N>
+    void run_visits(const double* dtemp, const uint8_t* sing, bool want_peaks) {
+        const int g = blocks_for(nel * (10 / N), 128, NUM_SMS * VISIT_BLOCKS);
+        if (want_peaks) peak.zero(s);
+        if (!want_peaks)
+            k_visit_strains<false, false, N><<<g, 128, 0, s>>>(
+                rec.p, mats.p, t10.p, u4.p, dtemp, sing, nel, nparts, visits.p, nullptr);
+        else if (nparts <= SMEM_PARTS)
+            k_visit_strains<true, true, N><<<g, 128, 3 * sizeof(u128) * nparts, s>>>(
+                rec.p, mats.p, t10.p, u4.p, dtemp, sing, nel, nparts, visits.p, peak.p);
+        else
+            k_visit_strains<true, false, N><<<g, 128, 0, s>>>(
+                rec.p, mats.p, t10.p, u4.p, dtemp, sing, nel, nparts, visits.p, peak.p);
     }
 
     void run(const double* u, const double* dtemp, double* stress, double* strain,
@@ -834,7 +1014,17 @@ struct femgpu_recovery {
             run_hex(dtemp, stress, strain, mises, principal, peaks, grid);
             return;
         }
-        if (!want_peaks) {
+        if (visits.p) {
+            // 10 visits per thread where the cells alone fill the device, else 2.
+            if (nel >= WHOLE_CELLS)
+                run_visits<10>(dtemp, sing, want_peaks);
+            else
+                run_visits<2>(dtemp, sing, want_peaks);
+            FG_CHECK_LAUNCH();
+            k_visit_means<<<grid, 128, 0, s>>>(visits.p, mats.p, inc.start.p, inc.of_node.p,
+                                               place.p, npoints, stress, strain, mises,
+                                               principal);
+        } else if (!want_peaks) {
             k_recover_points<false, false><<<grid, 128, 0, s>>>(
                 rec.p, mats.p, t10.p, inc.start.p, inc.of_node.p, place.p, u4.p, dtemp, sing,
                 npoints, nparts, stress, strain, mises, principal, nullptr);
@@ -996,6 +1186,14 @@ int femgpu_recovery_new(size_t npoints, const double* xyz, size_t nel, const uin
         r->mats.alloc(r->nmat);
         r->rec.alloc(nel);
         r->u4.alloc(4 * npoints);
+        if (80 * nel * sizeof(double) <= VISIT_BYTES_MAX) {
+            try {
+                r->visits.alloc(80 * nel);
+            } catch (const Failure&) {  // no room: the points evaluate their own visits
+                r->visits.release();
+                cudaGetLastError();
+            }
+        }
         DevBuf<int> bad(1);
         bad.zero(s);
         k_recover_materials<<<blocks_for(r->nmat, 128), 128, 0, s>>>(dtable.p, r->nmat, r->mats.p,
@@ -1213,7 +1411,7 @@ size_t femgpu_recovery_bytes(const femgpu_recovery* r) {
     if (!r) return 0;
     return r->t10.bytes() + r->rec.bytes() + r->mats.bytes() + r->singular.bytes() +
            r->hrec.bytes() + r->hmodes.bytes() + r->amp.bytes() +
-           r->place.bytes() + r->u4.bytes() + r->peak.bytes() + r->dpeaks.bytes() +
+           r->place.bytes() + r->u4.bytes() + r->visits.bytes() + r->peak.bytes() + r->dpeaks.bytes() +
            r->xyz.bytes() +
            r->inc.start.bytes() +
            r->inc.of_node.bytes() + r->du.bytes() + r->ddt.bytes() + r->dstress.bytes() +

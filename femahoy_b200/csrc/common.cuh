@@ -154,8 +154,15 @@ void exclusive_scan32(const uint32_t* in, int64_t* out, int64_t n, cudaStream_t 
 // the completion and the memory of the kernel before it, so it reads what it would have read
 // without the attribute. On the short kernels of the coarse levels the launch latency this
 // hides is most of their time.
-// (An explicit early trigger, griddepcontrol.launch_dependents after the wait, measured no
-// better on the 128^3 heat solve; the blocks trigger when they exit.)
+// (An explicit early trigger in the PCG kernels, whose inputs nothing can load ahead, measured no
+// better on the 128^3 heat solve and worse on a transient run, 6.47 -> 6.64 ms, and a batch, 22.0
+// -> 23.1 ms: those blocks trigger when they exit. The sparse solves trigger early.)
+// Lets the blocks of the kernel after this one start once every block of this one has called it
+// (or exited). For kernels that load much before their pdl_wait, and whose inputs the next kernel
+// reads by plain loads: the read-only path is for data that nothing writes while a kernel exists.
+__device__ __forceinline__ void pdl_trigger() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename... KArgs, typename... Args>

@@ -143,14 +143,20 @@ __global__ void __launch_bounds__(TH)
 // 17 us at the copy bandwidth), but a launch per level and direction leaves each level with a
 // few microseconds of dependent latency. So each task loads its first entries of G and its
 // static indices before it waits for the level before (programmatic dependent launch); after the
-// wait only 1 round of loads (the right side) comes before the sums. The children's updates are
+// wait only 1 round of loads (the right side) comes before the sums. A block lets the next level
+// start as soon as those loads are issued (`early`), so a level's launch and first loads run under
+// the levels before it; each still waits for the whole of the level before. The last backward
+// level does not: the kernel after it reads x through the read-only path, which must not change
+// while that kernel exists. (The trigger at the head of the kernel, before the loads: 541 us where
+// this takes 487; at the exit: 556.) The children's updates are
 // left in slots grouped by the parent's row, so that the parent reads them as 1 contiguous run.
 // Measured on B200: the 50 x 5 x 5 P2 beam's direct solve (2 applications of the factor, 36,300
 // unknowns) 3.70 -> 0.80 ms with 22 levels, 0.56 ms with the 11 levels of relaxed supernodes
-// (symbolic.cpp); the 29,910-unknown coarsest level of a prism mesh 1,633 -> 393 -> 199 us, its
-// kernels timed one by one. Before, 1 block took a whole supernode and the large ones near the
-// root left the other SMs idle. The error of 1 application against extended precision stayed:
-// 1e-12 to 6e-11 on P2 beams of 14,580 to 37,440 unknowns on either form.
+// (symbolic.cpp), 0.49 ms with the early trigger; the 29,910-unknown coarsest level of a prism
+// mesh 1,633 -> 393 -> 199 us, its kernels timed one by one (the early trigger takes 52 us more
+// off each iteration of that solve: 22.9 -> 21.0 ms). Before, 1 block took a whole supernode and
+// the large ones near the root left the other SMs idle. The error of 1 application against
+// extended precision stayed: 1e-12 to 6e-11 on P2 beams of 14,580 to 37,440 unknowns on any form.
 constexpr int SOLVE_WARPS = 16;
 constexpr int SOLVE_TH = 32 * SOLVE_WARPS;
 constexpr int ZCAP = 128;  // right side values staged per warp of a task
@@ -171,7 +177,7 @@ __global__ void __launch_bounds__(SOLVE_TH)
     k_sparse_forward(const SolveBlock* __restrict__ blocks, const SolveTask* __restrict__ tasks,
                      const double* __restrict__ G, const uint32_t* __restrict__ slot_ptr,
                      const uint32_t* __restrict__ dst, const int64_t* __restrict__ perm,
-                     const TB* b, double* slot, double* yf) {
+                     const TB* b, double* slot, double* yf, int early) {
     __shared__ double zs[SOLVE_WARPS * ZCAP];
     __shared__ double red[SOLVE_TH];
     const SolveBlock B = blocks[blockIdx.x];
@@ -203,6 +209,7 @@ __global__ void __launch_bounds__(SOLVE_TH)
         s1 = slot_ptr[t.z + row + 1];
         d = dst[t.z + row];
     }
+    if (early) pdl_trigger();
     pdl_wait();
     double acc = 0.0;
     // Tasks of fewer than 16 warps have at most `cap` columns: 1 turn for all of the block's.
@@ -263,7 +270,8 @@ __device__ __forceinline__ void backward_task(const SolveTask& t, int nw, int wg
                                               double* v, const double* __restrict__ G,
                                               const uint32_t* __restrict__ rows,
                                               const int64_t* __restrict__ perm,
-                                              const double* yf, double* xs, TX* x) {
+                                              const double* yf, double* xs, TX* x,
+                                              int early) {
     // Column c of the task is column at + c of G; W is lower triangular, so its rows above at
     // are 0.
     const int i0 = t.at & ~3;
@@ -285,6 +293,7 @@ __device__ __forceinline__ void backward_task(const SolveTask& t, int nw, int wg
     const int tid = wg * 32 + lane, gt = nw * 32, cap = ZCAP * nw;
     uint32_t r = 0;
     if (i0 + tid < t.m && i0 + tid >= t.k) r = rows[t.z + i0 + tid];
+    if (early) pdl_trigger();
     pdl_wait();
     // Tasks of fewer than 16 warps have at most `cap` rows: 1 turn for all of the block's.
     const int turns = nw == SOLVE_WARPS ? max(1, (t.m - i0 + cap - 1) / cap) : 1;
@@ -331,7 +340,8 @@ template <class TX>
 __global__ void __launch_bounds__(SOLVE_TH)
     k_sparse_backward(const SolveBlock* __restrict__ blocks, const SolveTask* __restrict__ tasks,
                       const double* __restrict__ G, const uint32_t* __restrict__ rows,
-                      const int64_t* __restrict__ perm, const double* yf, double* xs, TX* x) {
+                      const int64_t* __restrict__ perm, const double* yf, double* xs, TX* x,
+                      int early) {
     __shared__ double vs[SOLVE_WARPS * ZCAP];
     const SolveBlock B = blocks[blockIdx.x];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -340,11 +350,11 @@ __global__ void __launch_bounds__(SOLVE_TH)
     if (group < B.count) t = tasks[B.task + group];
     double* v = vs + group * ZCAP * nw;
     if (nw == 1)
-        backward_task<COLS_1, 2>(t, nw, wg, lane, v, G, rows, perm, yf, xs, x);
+        backward_task<COLS_1, 2>(t, nw, wg, lane, v, G, rows, perm, yf, xs, x, early);
     else if (nw == 4)
-        backward_task<COLS_4, 4>(t, nw, wg, lane, v, G, rows, perm, yf, xs, x);
+        backward_task<COLS_4, 4>(t, nw, wg, lane, v, G, rows, perm, yf, xs, x, early);
     else
-        backward_task<1, 8>(t, nw, wg, lane, v, G, rows, perm, yf, xs, x);
+        backward_task<1, 8>(t, nw, wg, lane, v, G, rows, perm, yf, xs, x, early);
 }
 
 // ---------------------------------------------------------------- the form of the solves
@@ -756,11 +766,11 @@ void SparseFactor::solve(const TB* b, TX* x, bool pdl, cudaStream_t s) {
     for (int64_t h = 0; h <= height_; ++h)
         launch(pdl, k_sparse_forward<TB>, (int)(forward_at_[h + 1] - forward_at_[h]), SOLVE_TH, s,
                forward_blocks_.p + forward_at_[h], forward_tasks_.p, g_.p, slot_ptr_.p, dst_.p,
-               perm_.p, b, slot_.p, y_.p);
+               perm_.p, b, slot_.p, y_.p, 1);
     for (int64_t h = height_; h >= 0; --h)
         launch(pdl, k_sparse_backward<TX>, (int)(backward_at_[h + 1] - backward_at_[h]), SOLVE_TH,
                s, backward_blocks_.p + backward_at_[h], backward_tasks_.p, g_.p, rows_.p, perm_.p,
-               y_.p, xs_.p, x);
+               y_.p, xs_.p, x, h > 0 ? 1 : 0);
 }
 template void SparseFactor::solve<double, double>(const double*, double*, bool, cudaStream_t);
 template void SparseFactor::solve<float, float>(const float*, float*, bool, cudaStream_t);

@@ -4,7 +4,7 @@
 // two triangular solves.
 //
 // Layout. Each supernode s owns a dense frontal matrix F_s of m_s x m_s doubles (column-major,
-// its rows R_s), kept for the solves: its first k_s columns become the columns of L, and its
+// its rows R_s) while it is factored: its first k_s columns become the columns of L, and its
 // trailing block is the update matrix (Schur complement) that its parent takes. The entries of A
 // are scattered into all fronts at once; then the fronts are done level by level in the
 // supernode tree (height 0 = leaves), so every child is factored before its parent:

@@ -1496,7 +1496,7 @@ def run_recover(opt, rank, world, local):
                      "frac": achieved / peak, "peak_kind": peak_kind,
                      "kernel": ("k_pad_u + k_hex_amplitudes + k_recover_hex_points<peaks> + "
                                 "k_peak_final" if hexes else
-                                "k_pad_u + k_recover_points<peaks> + k_peak_final"),
+                                "k_pad_u + k_visit_strains + k_visit_means + k_peak_final"),
                      "bytes_per_launch": kbytes, "launch_ms": kernel_ms, "traffic": None},
         "cpu_baseline": cpu,
         "e2e": {"value": e2e_value, "unit": "points/s", "h2d_bytes_per_step": 24 * n,

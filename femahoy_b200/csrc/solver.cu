@@ -3376,17 +3376,18 @@ void SolverImpl::solve(const double* d_b, double* d_x, const volatile int* cance
     }
     // multigrid.rs:692-753
     if (d_x != x_.p) FG_CUDA(cudaMemcpyAsync(x_.p, d_x, n * 8, cudaMemcpyDeviceToDevice, s_));
-    if (opt_.graph && !exec_) {
-        build_graph();
-        graph_tol_ = tol;
-    }
-    // The graph's stopping test keeps the tolerance of the solve that captured it.
-    if (exec_) h_init_->tol = graph_tol_;
+    if (opt_.graph && !exec_) build_graph();
     int status = FEMGPU_OK;
     std::string message;
     double residual = 0.0;
     size_t it = 0;
-    for (int restarts = 0;;) {
+    // The FP64 form takes the recurrence's residual for the residual, as the reference does. But a
+    // recurrence whose r.r underflowed to 0 has lost r (a tolerance of 1e-300, which nothing else
+    // meets), so the solve goes on from x's own residual while iterations are left; then x
+    // is taken as it is.
+    bool lost = false;
+    for (int restarts = 0, idle = 0;;) {
+        const size_t before = it;
         h_init_->iters = (int)std::min<size_t>(it, 0x7fffffff);
         if (exec_)
             run_graph(cancel);
@@ -3413,9 +3414,15 @@ void SolverImpl::solve(const double* d_b, double* d_x, const volatile int* cance
             // from it, and then the solve restarts from x (iterative refinement).
             const double truth = std::sqrt(h_sc_->truth) / norm_b;
             out.true_residual = truth;
-            if (truth <= tol || !mixed || restarts >= 3 || it >= max_iter) break;
+            lost = lost || (!mixed && h_sc_->rr == 0.0 && tol > 0.0);
+            if (truth <= tol || it >= max_iter || !(mixed ? restarts < 3 : lost)) break;
+            if (restarts > 0 && it == before) break;  // nothing changes from here
             ++restarts;
             continue;
+        }
+        if (it >= max_iter && lost) {
+            out.true_residual = std::sqrt(h_sc_->truth) / norm_b;
+            break;
         }
         if (it >= max_iter) {
             char buf[200];
@@ -3430,6 +3437,13 @@ void SolverImpl::solve(const double* d_b, double* d_x, const volatile int* cance
         if (cancel && *cancel) {
             status = FEMGPU_ERR_CANCELLED;
             message = "cancelled";
+            break;
+        }
+        // Only a flag that was raised and taken back ends a run here; a run that does nothing time
+        // and again must not go on for ever.
+        if (it == before && ++idle == 3) {
+            status = FEMGPU_ERR_NOT_CONVERGED;
+            message = "conjugate gradients made no iteration";
             break;
         }
     }

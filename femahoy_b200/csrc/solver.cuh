@@ -358,7 +358,6 @@ class SolverImpl {
     std::vector<std::pair<std::string, double>> setup_s_;
     size_t launches_ = 0;      // kernels enqueued by the current solve
     bool in_graph_ = false;    // while the solve's graph is captured
-    double graph_tol_ = 0;     // the tolerance the graph was captured for
     // The kernels of the graph: its start and end, and 1 iteration.
     size_t fixed_kernels_ = 0, loop_kernels_ = 0;
 };

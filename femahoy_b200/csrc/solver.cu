@@ -2141,8 +2141,7 @@ SolverImpl::SolverImpl() {
 
 SolverImpl::~SolverImpl() {
     if (l2_window_) cudaCtxResetPersistingL2Cache();
-    if (exec_) cudaGraphExecDestroy(exec_);
-    if (graph_) cudaGraphDestroy(graph_);
+    drop_graphs();
     if (h_sc_) cudaFreeHost(h_sc_);
     if (h_cancel_) cudaFreeHost(h_cancel_);
     if (ev0_) cudaEventDestroy(ev0_);
@@ -2388,11 +2387,7 @@ void SolverImpl::apply_degree(int degree, int coarse) {
     for (size_t l = 0; l < H64_.levels.size(); ++l)
         chebyshev(H64_.levels[l].lambda, l == 0 ? degree : coarse, lower, &H64_.levels[l].c1,
                   &H64_.levels[l].c2, opt_.smoother, opt_.upper);
-    // The captured loop holds the coefficients as kernel arguments.
-    if (exec_) cudaGraphExecDestroy(exec_);
-    if (graph_) cudaGraphDestroy(graph_);
-    exec_ = nullptr;
-    graph_ = nullptr;
+    drop_graphs();  // the captured loops hold the coefficients as kernel arguments
 }
 
 // Each candidate (the finest level's degree, the coarser levels') solves a fixed right side
@@ -3075,15 +3070,30 @@ void SolverImpl::enqueue_cycle(Hierarchy<T>& H, const T* r, bool started, bool i
     launches_ += 2;
 }
 
-// The start of a solve from x: r = b - A x, and the first p.
-void SolverImpl::enqueue_start() {
+// r = b - A x, and its FP32 copy to r32 if set, with the sums b.b and r.r; the blocks launched.
+// `exact`: by the operator that holds every entry of the matrix.
+int SolverImpl::enqueue_pcg_residual(bool exact, bool pdl, double* r, float* r32) {
+    if (exact && op64_.stencil) {
+        const int nb = row_blocks(A64_.nslices * A64_.C);
+        launch(pdl, k_pcg_residual<SellOp<double>>, nb, TH, s_, SellOp<double>{A64_.view()}, b_.p,
+               x_.p, r, r32, partial_.p);
+        return nb;
+    }
+    const int nb = row_blocks(op64_.threads());
+    with_op(op64_, [&](auto op) {
+        launch(pdl, k_pcg_residual<decltype(op)>, nb, TH, s_, op, b_.p, x_.p, r, r32,
+               partial_.p);
+    });
+    return nb;
+}
+
+// The start of a solve from x: r = b - A x, and the first p. `restart`: r as the true residual
+// that called for it has it, by the exact matrix. (A stencil takes the lower triangle from the upper
+// one; where they differ, its own residual can be at the tolerance and the true one above.)
+void SolverImpl::enqueue_start(bool restart) {
     const bool mixed = opt_.precision == FEMGPU_MIXED;
     FG_CUDA(cudaMemcpyAsync(sc_.p, h_init_, sizeof(Scalars), cudaMemcpyHostToDevice, s_));
-    const int nbq = row_blocks(op64_.threads());
-    with_op(op64_, [&](auto op) {
-        launch(false, k_pcg_residual<decltype(op)>, nbq, TH, s_, op, b_.p, x_.p, r_.p,
-               mixed ? r32_.p : nullptr, partial_.p);
-    });
+    const int nbq = enqueue_pcg_residual(restart, false, r_.p, mixed ? r32_.p : nullptr);
     launch(pdl_, k_finish<FinStart>, 1, FIN_TH, s_, partial_.p, nbq, FinStart{sc_.p});
     FG_CHECK_LAUNCH();
     launches_ += 2;
@@ -3123,18 +3133,9 @@ void SolverImpl::enqueue_iteration() {
         rest(H64_, r_.p, (float*)nullptr);
 }
 
-// The true residual of x, by the operator that holds every entry of the matrix.
+// The true residual of x.
 void SolverImpl::enqueue_truth() {
-    const bool sell = op64_.stencil;
-    const int nb = sell ? row_blocks(A64_.nslices * A64_.C) : row_blocks(op64_.threads());
-    if (sell)
-        launch(pdl_, k_pcg_residual<SellOp<double>>, nb, TH, s_, SellOp<double>{A64_.view()},
-               b_.p, x_.p, t_.p, (float*)nullptr, partial_.p);
-    else
-        with_op(op64_, [&](auto op) {
-            launch(pdl_, k_pcg_residual<decltype(op)>, nb, TH, s_, op, b_.p, x_.p, t_.p,
-                   (float*)nullptr, partial_.p);
-        });
+    const int nb = enqueue_pcg_residual(true, pdl_, t_.p, nullptr);
     launch(pdl_, k_finish<FinTruth>, 1, FIN_TH, s_, partial_.p, nb, FinTruth{sc_.p});
     FG_CHECK_LAUNCH();
     launches_ += 2;
@@ -3146,18 +3147,19 @@ void SolverImpl::enqueue_truth() {
 // round trip. (With the start and the true residual as stream launches around the loop's graph, a
 // solve waited for the device 4 times: 118 of the 188 us of the 3,000 unknown cantilever, 155 of
 // 755 us at 110,544 unknowns.)
-void SolverImpl::build_graph() {
+void SolverImpl::build_graph(bool restart) {
+    SolveGraph& G = graphs_[restart];
     for (;;) {
         const size_t before = launches_;
         try {
-            FG_CUDA(cudaGraphCreate(&graph_, 0));
-            FG_CUDA(cudaGraphConditionalHandleCreate(&cond_, graph_, 0,
+            FG_CUDA(cudaGraphCreate(&G.graph, 0));
+            FG_CUDA(cudaGraphConditionalHandleCreate(&cond_, G.graph, 0,
                                                      cudaGraphCondAssignDefault));
             in_graph_ = true;
-            FG_CUDA(cudaStreamBeginCaptureToGraph(s_, graph_, nullptr, nullptr, 0,
+            FG_CUDA(cudaStreamBeginCaptureToGraph(s_, G.graph, nullptr, nullptr, 0,
                                                   cudaStreamCaptureModeThreadLocal));
-            enqueue_start();
-            fixed_kernels_ = launches_ - before;
+            enqueue_start(restart);
+            G.fixed_kernels = launches_ - before;
             cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
             const cudaGraphNode_t* at = nullptr;
             size_t count = 0;
@@ -3171,21 +3173,21 @@ void SolverImpl::build_graph() {
             cp.conditional.type = cudaGraphCondTypeWhile;
             cp.conditional.size = 1;
             cudaGraphNode_t node;
-            FG_CUDA(cudaGraphAddNode(&node, graph_, last.data(), last.size(), &cp));
+            FG_CUDA(cudaGraphAddNode(&node, G.graph, last.data(), last.size(), &cp));
             cudaGraph_t body = cp.conditional.phGraph_out[0];
             launches_ = before;
             FG_CUDA(cudaStreamBeginCaptureToGraph(s_, body, nullptr, nullptr, 0,
                                                   cudaStreamCaptureModeThreadLocal));
             enqueue_iteration();
             FG_CUDA(cudaStreamEndCapture(s_, &same));
-            loop_kernels_ = launches_ - before;
+            G.loop_kernels = launches_ - before;
             launches_ = before;
-            FG_CUDA(cudaStreamBeginCaptureToGraph(s_, graph_, &node, nullptr, 1,
+            FG_CUDA(cudaStreamBeginCaptureToGraph(s_, G.graph, &node, nullptr, 1,
                                                   cudaStreamCaptureModeThreadLocal));
             enqueue_truth();
             FG_CUDA(cudaStreamEndCapture(s_, &same));
-            fixed_kernels_ += launches_ - before;
-            FG_CUDA(cudaGraphInstantiate(&exec_, graph_, 0));
+            G.fixed_kernels += launches_ - before;
+            FG_CUDA(cudaGraphInstantiate(&G.exec, G.graph, 0));
             in_graph_ = false;
             launches_ = before;
             return;
@@ -3200,10 +3202,7 @@ void SolverImpl::build_graph() {
                 cudaStreamEndCapture(s_, &g);
             }
             cudaGetLastError();
-            if (exec_) cudaGraphExecDestroy(exec_);
-            if (graph_) cudaGraphDestroy(graph_);
-            exec_ = nullptr;
-            graph_ = nullptr;
+            G.drop();
             launches_ = before;
             // Give up the fused coarse levels first, then the cluster legs, then the
             // programmatic launches.
@@ -3225,14 +3224,13 @@ void SolverImpl::build_graph() {
 
 void SolverImpl::set_wait_limit(unsigned polls) {
     wait_limit = polls;
-    if (exec_) cudaGraphExecDestroy(exec_);
-    if (graph_) cudaGraphDestroy(graph_);
-    exec_ = nullptr;
-    graph_ = nullptr;
+    drop_graphs();
 }
 
-// Runs the solve's graph; *h_sc_ holds the scalars when it returns.
-void SolverImpl::run_graph(const volatile int* cancel) {
+// Runs a solve's graph; *h_sc_ holds the scalars when it returns.
+void SolverImpl::run_graph(bool restart, const volatile int* cancel) {
+    if (!graphs_[restart].exec) build_graph(restart);
+    const SolveGraph& G = graphs_[restart];
     *(volatile int*)h_cancel_ = cancel && *cancel ? 1 : 0;
     std::atomic<bool> stop{false};
     std::thread watcher;
@@ -3246,21 +3244,21 @@ void SolverImpl::run_graph(const volatile int* cancel) {
         });
     }
     const int before = h_init_->iters;
-    cudaError_t e = cudaGraphLaunch(exec_, s_);
+    cudaError_t e = cudaGraphLaunch(G.exec, s_);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s_);
     stop.store(true);
     if (watcher.joinable()) watcher.join();
     FG_CUDA(e);
-    launches_ += fixed_kernels_ + loop_kernels_ * (size_t)(h_sc_->iters - before);
+    launches_ += G.fixed_kernels + G.loop_kernels * (size_t)(h_sc_->iters - before);
 }
 
 // The same with every kernel its own launch (option graph = 2).
-void SolverImpl::run_launches(const volatile int* cancel) {
+void SolverImpl::run_launches(bool restart, const volatile int* cancel) {
     auto scalars = [&] {
         FG_CUDA(cudaMemcpyAsync(h_sc_, sc_.p, sizeof(Scalars), cudaMemcpyDeviceToHost, s_));
         FG_CUDA(cudaStreamSynchronize(s_));
     };
-    enqueue_start();
+    enqueue_start(restart);
     scalars();
     while (!h_sc_->done && h_sc_->iters < h_sc_->max_iter && h_sc_->rr == h_sc_->rr &&
            !h_sc_->bulk_timeout && !(cancel && *cancel)) {
@@ -3376,7 +3374,6 @@ void SolverImpl::solve(const double* d_b, double* d_x, const volatile int* cance
     }
     // multigrid.rs:692-753
     if (d_x != x_.p) FG_CUDA(cudaMemcpyAsync(x_.p, d_x, n * 8, cudaMemcpyDeviceToDevice, s_));
-    if (opt_.graph && !exec_) build_graph();
     int status = FEMGPU_OK;
     std::string message;
     double residual = 0.0;
@@ -3389,10 +3386,11 @@ void SolverImpl::solve(const double* d_b, double* d_x, const volatile int* cance
     for (int restarts = 0, idle = 0;;) {
         const size_t before = it;
         h_init_->iters = (int)std::min<size_t>(it, 0x7fffffff);
-        if (exec_)
-            run_graph(cancel);
+        const bool exact = restarts > 0 && op64_.stencil;
+        if (opt_.graph)
+            run_graph(exact, cancel);
         else
-            run_launches(cancel);
+            run_launches(exact, cancel);
         const double norm_b = h_sc_->norm_b;
         if (norm_b == 0.0) {
             FG_CUDA(cudaMemsetAsync(d_x, 0, n * 8, s_));

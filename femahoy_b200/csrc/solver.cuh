@@ -303,14 +303,18 @@ class SolverImpl {
     void enqueue_residual(MgLevel<T>& L, const T* b, const T* x);
     template <class T>
     void enqueue_cycle(Hierarchy<T>& H, const T* r, bool started, bool init);
-    void enqueue_start();
+    int enqueue_pcg_residual(bool exact, bool pdl, double* r, float* r32);
+    void enqueue_start(bool restart);
     void enqueue_iteration();
     void enqueue_truth();
     void enqueue_spmv_pq();
-    void build_graph();
+    void build_graph(bool restart);
     // Solve from x_ until convergence, max_iter, a NaN or a cancel.
-    void run_graph(const volatile int* cancel);
-    void run_launches(const volatile int* cancel);
+    void run_graph(bool restart, const volatile int* cancel);
+    void run_launches(bool restart, const volatile int* cancel);
+    void drop_graphs() {
+        for (SolveGraph& g : graphs_) g.drop();
+    }
     void dense_direct(const HostCsr& a);
     // The Chebyshev degree of every level (1, 2 or 3) by timed trial solves, per size class.
     void tune_degree();
@@ -340,9 +344,20 @@ class SolverImpl {
     Scalars* h_sc_ = nullptr;    // pinned: the scalars of the last solve
     Scalars* h_init_ = nullptr;  // pinned: what a solve starts from
     DevBuf<int> done_zero_;
-    cudaGraph_t graph_ = nullptr;
-    cudaGraphExec_t exec_ = nullptr;
-    cudaGraphConditionalHandle cond_ = 0;
+    // A solve as 1 graph, with the kernels of its start and end, and of 1 iteration.
+    struct SolveGraph {
+        cudaGraph_t graph = nullptr;
+        cudaGraphExec_t exec = nullptr;
+        size_t fixed_kernels = 0, loop_kernels = 0;
+        void drop() {
+            if (exec) cudaGraphExecDestroy(exec);
+            if (graph) cudaGraphDestroy(graph);
+            exec = nullptr;
+            graph = nullptr;
+        }
+    };
+    SolveGraph graphs_[2];  // of a solve; of a restart by the exact matrix (made when one is due)
+    cudaGraphConditionalHandle cond_ = 0;  // the loop of the graph being captured
     int* h_cancel_ = nullptr;  // pinned and mapped: the device reads it each iteration
     int* d_cancel_ = nullptr;
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
@@ -357,9 +372,7 @@ class SolverImpl {
     // Seconds of each phase of the setup, in the order first met (reported by describe()).
     std::vector<std::pair<std::string, double>> setup_s_;
     size_t launches_ = 0;      // kernels enqueued by the current solve
-    bool in_graph_ = false;    // while the solve's graph is captured
-    // The kernels of the graph: its start and end, and 1 iteration.
-    size_t fixed_kernels_ = 0, loop_kernels_ = 0;
+    bool in_graph_ = false;    // while a solve's graph is captured
 };
 
 }  // namespace femgpu

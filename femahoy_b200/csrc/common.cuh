@@ -57,13 +57,15 @@ inline int blocks_for(int64_t n, int threads, int cap = NUM_SMS * 16) {
 // scope's stream alone until it has been synchronized, and every buffer that outlives the scope
 // is handed on after that. A pooled buffer freed with no scope open is returned at once: its
 // owner has then synchronized the streams that used it (the solver's destructor its own stream;
-// every call on a matrix synchronizes before it returns, on errors too). The pool keeps 2 GiB at
-// most, gives them back when an allocation does not fit or a server makes room, and its order
-// across streams and threads is the CUDA runtime's own.
+// every call on a matrix synchronizes before it returns, on errors too). Outside scopes the pool
+// keeps 2 GiB of free memory at most (while one is open, all that it has: a setup frees and asks
+// again and again), gives them back when an allocation does not fit, when a server makes room or
+// when the caller asks (femgpu_trim), and its order across streams and threads is the CUDA
+// runtime's own.
 class PoolScope {
    public:
-    explicit PoolScope(cudaStream_t s) : s_(s), outer_(current_) { current_ = this; }
-    ~PoolScope() { current_ = outer_; }
+    explicit PoolScope(cudaStream_t s);
+    ~PoolScope();
     PoolScope(const PoolScope&) = delete;
     PoolScope& operator=(const PoolScope&) = delete;
     cudaStream_t stream() const { return s_; }
@@ -71,13 +73,14 @@ class PoolScope {
 
    private:
     cudaStream_t s_;
+    int device_ = -1;
     const PoolScope* outer_;
     static inline thread_local const PoolScope* current_ = nullptr;
 };
 
-// `pooled` tells device_free how the memory was made.
-cudaError_t device_alloc(void** p, size_t bytes, bool* pooled);
-void device_free(void* p, bool pooled);
+// `pool` tells device_free where the memory came from: the device whose pool it was, or -1.
+cudaError_t device_alloc(void** p, size_t bytes, int* pool);
+void device_free(void* p, size_t bytes, int pool);
 // Gives what the current device's pool keeps free back to the device.
 void pool_trim();
 
@@ -86,12 +89,12 @@ template <class T>
 struct DevBuf {
     T* p = nullptr;
     size_t count = 0;
-    bool pooled = false;
+    int pool = -1;  // of the device whose pool p is from
     DevBuf() = default;
     explicit DevBuf(size_t n) { alloc(n); }
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
-    DevBuf(DevBuf&& o) noexcept : p(o.p), count(o.count), pooled(o.pooled) {
+    DevBuf(DevBuf&& o) noexcept : p(o.p), count(o.count), pool(o.pool) {
         o.p = nullptr;
         o.count = 0;
     }
@@ -100,7 +103,7 @@ struct DevBuf {
             release();
             p = o.p;
             count = o.count;
-            pooled = o.pooled;
+            pool = o.pool;
             o.p = nullptr;
             o.count = 0;
         }
@@ -110,10 +113,10 @@ struct DevBuf {
     void alloc(size_t n) {
         release();
         count = n;
-        if (n) FG_CUDA(device_alloc((void**)&p, n * sizeof(T), &pooled));
+        if (n) FG_CUDA(device_alloc((void**)&p, n * sizeof(T), &pool));
     }
     void release() {
-        if (p) device_free(p, pooled);
+        if (p) device_free(p, count * sizeof(T), pool);
         p = nullptr;
         count = 0;
     }

@@ -1,0 +1,50 @@
+"""What the setup buffers' pool keeps: free blocks stay for the next setup however much is in use, and
+at most 2 GiB of them once the buffers are freed."""
+import gc
+
+import numpy as np
+import pytest
+
+import femahoy_b200 as fg
+from femahoy_b200 import meshgen as mg
+
+pytestmark = pytest.mark.gpu
+
+GIB = 2**30
+
+
+def _free():
+    import torch
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+def _matrices(k, rows, bytes_):
+    """Device copies of k that hold about ``bytes_`` in all."""
+    n, nnz = k.shape
+    each = 12 * nnz + 8 * (n + 1)
+    return [k.submatrix(rows) for _ in range(-(-bytes_ // each))]
+
+
+def test_free_blocks_stay_beside_a_large_user_and_are_bounded():
+    h = mg.heat_cube(64)
+    k = fg.Csr.assemble(fg.P1_HEAT, h.xyz, h.nodes, h.coef)
+    rows = np.arange(k.shape[0])
+    k.submatrix(rows)
+    gc.collect()
+    start = _free()
+    held = _matrices(k, rows, 3 * GIB)
+    before = _free()
+    more = _matrices(k, rows, GIB // 2)
+    with_more = _free()
+    assert before - with_more <= GIB  # the pool grows by what is asked for
+    del more
+    gc.collect()
+    # Freed beside 3 GiB in use: kept for the next setup (a fixed threshold gave them back here).
+    assert _free() - with_more <= GIB // 8
+    again = _matrices(k, rows, GIB // 2)
+    assert with_more - _free() <= GIB // 8
+    # All freed: 2 GiB kept at most (blocks are whole pieces of memory of a few MiB).
+    del held, again
+    gc.collect()
+    assert start - _free() <= 2 * GIB + GIB // 8

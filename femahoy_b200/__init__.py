@@ -9,7 +9,7 @@ The Python names mirror the reference crate: ``Csr`` (sparse.rs), ``Solver``, ``
 meshes (prism.rs, mesh2d.rs) and ``grid`` its box grid (grid.rs Grid::build).
 """
 from ._lib import (COLOUR, FP64, GATHER, HEX8_ELASTIC, HEX8_HEAT, HEX8_MASS, MIXED, P1_ELASTIC, P1_HEAT, P2_ELASTIC,
-                   P2_ELASTIC_ORTHO, P2_MASS, FemError, LIB_PATH, lib)
+                   P2_ELASTIC_ORTHO, P2_MASS, FemError, LIB_PATH, lib, trim)
 from .solve import (PCG_MAX_ITER, PCG_TOL, STEADY_DIRECT_LIMIT, TRANSIENT_DIRECT_LIMIT,
                     Cells, Convergence, Crossover, Level, Method, Options, Quadratic, Solver,
                     Stats, Unknowns, coarse_matrix, hex_elements, hex_mass, pcg, prolongation,
@@ -21,7 +21,7 @@ from . import grid, prism
 __all__ = [
     "COLOUR", "FP64", "GATHER", "HEX8_ELASTIC", "HEX8_HEAT", "HEX8_MASS", "MIXED", "P1_ELASTIC", "P1_HEAT", "P2_ELASTIC", "P2_ELASTIC_ORTHO", "P2_MASS",
     "FemError",
-    "LIB_PATH", "lib", "PCG_MAX_ITER", "PCG_TOL", "STEADY_DIRECT_LIMIT",
+    "LIB_PATH", "lib", "trim", "PCG_MAX_ITER", "PCG_TOL", "STEADY_DIRECT_LIMIT",
     "TRANSIENT_DIRECT_LIMIT", "Cells", "Crossover", "Level", "Method", "Options", "Quadratic",
     "Solver", "coarse_matrix", "hex_elements", "hex_mass", "symbolic_counts",
     "Stats", "Unknowns", "prolongation", "reduced_rhs", "Csr", "Rect", "colour", "Peak",

@@ -175,6 +175,7 @@ SIGNATURES = {
     "femgpu_boxgrid_free": (None, [C.c_void_p]),
     "femgpu_last_error": (C.c_size_t, [C.c_char_p, C.c_size_t]),
     "femgpu_version": (C.c_char_p, []),
+    "femgpu_trim": (C.c_int, []),
     "femgpu_assemble": (C.c_int, [C.c_int, C.c_int, C.c_size_t, C.c_void_p, C.c_size_t,
                                   C.c_void_p, C.c_void_p, C.POINTER(C.c_void_p)]),
     "femgpu_assemble_device": (C.c_int, [C.c_int, C.c_int, C.c_size_t, C.c_void_p, C.c_size_t,
@@ -336,6 +337,12 @@ def check(status):
         buf = C.create_string_buffer(1024)
         lib().femgpu_last_error(buf, 1024)
         raise FemError(status, buf.value.decode())
+
+
+def trim():
+    """Gives the free device memory that the library keeps for its next setup (at most 2 GiB) back to
+    the device, for another allocator of the process."""
+    check(lib().femgpu_trim())
 
 
 def ptr(a):

@@ -67,6 +67,10 @@ size_t femgpu_last_error(char* buf, size_t len) {
 
 const char* femgpu_version(void) { return "femgpu 0.1 (sm_100a)"; }
 
+int femgpu_trim(void) {
+    return guarded([] { pool_trim(); });
+}
+
 static int assemble_impl(int kind, int mode, size_t npoints, const double* xyz, size_t nel,
                          const uint32_t* nodes, const double* coef, femgpu_csr** out,
                          bool device) {

@@ -89,6 +89,10 @@ typedef struct femgpu_solver femgpu_solver; /* solve.rs:58-61 `Solver` */
 size_t femgpu_last_error(char* buf, size_t len);
 /* The library version and the device it runs on. */
 const char* femgpu_version(void);
+/* Gives the free device memory that the library keeps for its next setup (at most 2 GiB on the
+ * current device, outside calls) back to the device. The library does so itself when one of its own
+ * allocations does not fit; another allocator of the process (PyTorch's, say) calls this. */
+int femgpu_trim(void);
 
 /* ---------------------------------------------------------------- assembly */
 

@@ -48,3 +48,19 @@ def test_free_blocks_stay_beside_a_large_user_and_are_bounded():
     del held, again
     gc.collect()
     assert start - _free() <= 2 * GIB + GIB // 8
+
+
+def test_trim_gives_the_free_memory_back():
+    h = mg.heat_cube(48)
+    k = fg.Csr.assemble(fg.P1_HEAT, h.xyz, h.nodes, h.coef)
+    rows = np.arange(k.shape[0])
+    k.submatrix(rows)
+    gc.collect()
+    fg.trim()
+    start = _free()
+    held = _matrices(k, rows, GIB)
+    del held
+    gc.collect()
+    assert start - _free() >= GIB // 2  # kept for the next setup
+    fg.trim()
+    assert start - _free() <= GIB // 16

@@ -308,6 +308,7 @@ SIGNATURES = {
                                       C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "femgpu_recovery_run_device": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
                                              C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
+    "femgpu_recovery_set_scratch": (C.c_int, [C.c_void_p, C.c_size_t]),
     "femgpu_recovery_last_time": (C.c_int, [C.c_void_p, C.POINTER(C.c_double),
                                             C.POINTER(C.c_double)]),
     "femgpu_recovery_bytes": (C.c_size_t, [C.c_void_p]),

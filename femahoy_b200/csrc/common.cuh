@@ -64,7 +64,9 @@ inline int blocks_for(int64_t n, int threads, int cap = NUM_SMS * 16) {
 // runtime's own.
 class PoolScope {
    public:
-    explicit PoolScope(cudaStream_t s);
+    // `setup` false: a run of a handle, whose buffers are few and alike from call to call, so that
+    // what the pool keeps need not be touched.
+    explicit PoolScope(cudaStream_t s, bool setup = true);
     ~PoolScope();
     PoolScope(const PoolScope&) = delete;
     PoolScope& operator=(const PoolScope&) = delete;

@@ -65,8 +65,9 @@ cudaMemPool_t pool_of(int device) {
 
 }  // namespace
 
-PoolScope::PoolScope(cudaStream_t s) : s_(s), outer_(current_) {
+PoolScope::PoolScope(cudaStream_t s, bool setup) : s_(s), outer_(current_) {
     current_ = this;
+    if (!setup) return;
     int device = 0;
     if (cudaGetDevice(&device) != cudaSuccess) return;
     Pool* e = entry(device);

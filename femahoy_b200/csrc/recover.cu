@@ -24,7 +24,8 @@
 // set the time: 531 us for the 160 x 20 x 20 P2 beam (384,000 cells, 3.84M visits; the 3 largest
 // kernels by CUDA events 482), now 283 (180 for the visits, 96 for the means); 239 -> 51 us for
 // 15,360 cells, where each block also raised its parts' maxima from nothing.
-// That form serves meshes whose visits would take more than VISIT_BYTES_MAX.
+// That form serves meshes whose visits would take more than VISIT_BYTES_MAX, callers that give
+// less, and devices with no room for them.
 //
 // Peaks: the thread of each visit folds its von Mises stress into 3 running maxima of its part,
 // each a 128-bit word updated by compare-and-swap: (value, ~key) for the peak and for the
@@ -403,7 +404,7 @@ __device__ __forceinline__ void write_point(int64_t v, int64_t count, double ss[
     }
 }
 
-// The most that the visits' 64 bytes may take.
+// The most that the visits' 64 bytes may take unless the caller sets it.
 constexpr size_t VISIT_BYTES_MAX = (size_t)4 << 30;
 // From this many cells on a thread takes all 10 visits of a cell.
 constexpr int64_t WHOLE_CELLS = 100'000;
@@ -973,7 +974,7 @@ struct femgpu_recovery {
     DevBuf<MaterialEntry> mats;
     DevBuf<uint8_t> singular;
     DevBuf<double> u4;
-    DevBuf<double> visits;  // 8 per visit; empty where they would take too much memory
+    size_t visit_limit = VISIT_BYTES_MAX;  // the most that a run's visits may take
     DevBuf<u128> peak;
     DevBuf<femgpu_peak> dpeaks;
     // Device copies for the host-pointer form.
@@ -987,19 +988,31 @@ struct femgpu_recovery {
         if (s) cudaStreamDestroy(s);
     }
 
+    // The visits of a run, or nothing. They are scratch of that run alone, from the pool: kept in
+    // the handle they would take the room of what the caller makes next.
+    void take_visits(DevBuf<double>* v) const {
+        if (80 * (size_t)nel * sizeof(double) > visit_limit) return;
+        try {
+            v->alloc(80 * (size_t)nel);
+        } catch (const Failure&) {  // no room: the points evaluate their own visits
+            v->release();
+            cudaGetLastError();
+        }
+    }
+
     template <int N>
-    void run_visits(const double* dtemp, const uint8_t* sing, bool want_peaks) {
+    void run_visits(const double* dtemp, const uint8_t* sing, bool want_peaks, double* visits) {
         const int g = blocks_for(nel * (10 / N), 128, NUM_SMS * VISIT_BLOCKS);
         if (want_peaks) peak.zero(s);
         if (!want_peaks)
             k_visit_strains<false, false, N><<<g, 128, 0, s>>>(
-                rec.p, mats.p, t10.p, u4.p, dtemp, sing, nel, nparts, visits.p, nullptr);
+                rec.p, mats.p, t10.p, u4.p, dtemp, sing, nel, nparts, visits, nullptr);
         else if (nparts <= SMEM_PARTS)
             k_visit_strains<true, true, N><<<g, 128, 3 * sizeof(u128) * nparts, s>>>(
-                rec.p, mats.p, t10.p, u4.p, dtemp, sing, nel, nparts, visits.p, peak.p);
+                rec.p, mats.p, t10.p, u4.p, dtemp, sing, nel, nparts, visits, peak.p);
         else
             k_visit_strains<true, false, N><<<g, 128, 0, s>>>(
-                rec.p, mats.p, t10.p, u4.p, dtemp, sing, nel, nparts, visits.p, peak.p);
+                rec.p, mats.p, t10.p, u4.p, dtemp, sing, nel, nparts, visits, peak.p);
     }
 
     void run(const double* u, const double* dtemp, double* stress, double* strain,
@@ -1014,12 +1027,15 @@ struct femgpu_recovery {
             run_hex(dtemp, stress, strain, mises, principal, peaks, grid);
             return;
         }
+        PoolScope pool(s, false);
+        DevBuf<double> visits;
+        take_visits(&visits);
         if (visits.p) {
             // 10 visits per thread where the cells alone fill the device, else 2.
             if (nel >= WHOLE_CELLS)
-                run_visits<10>(dtemp, sing, want_peaks);
+                run_visits<10>(dtemp, sing, want_peaks, visits.p);
             else
-                run_visits<2>(dtemp, sing, want_peaks);
+                run_visits<2>(dtemp, sing, want_peaks, visits.p);
             FG_CHECK_LAUNCH();
             k_visit_means<<<grid, 128, 0, s>>>(visits.p, mats.p, inc.start.p, inc.of_node.p,
                                                place.p, npoints, stress, strain, mises,
@@ -1186,14 +1202,6 @@ int femgpu_recovery_new(size_t npoints, const double* xyz, size_t nel, const uin
         r->mats.alloc(r->nmat);
         r->rec.alloc(nel);
         r->u4.alloc(4 * npoints);
-        if (80 * nel * sizeof(double) <= VISIT_BYTES_MAX) {
-            try {
-                r->visits.alloc(80 * nel);
-            } catch (const Failure&) {  // no room: the points evaluate their own visits
-                r->visits.release();
-                cudaGetLastError();
-            }
-        }
         DevBuf<int> bad(1);
         bad.zero(s);
         k_recover_materials<<<blocks_for(r->nmat, 128), 128, 0, s>>>(dtable.p, r->nmat, r->mats.p,
@@ -1212,6 +1220,12 @@ int femgpu_recovery_new(size_t npoints, const double* xyz, size_t nel, const uin
         r->peak.alloc(3 * nparts);
         r->dpeaks.alloc(nparts);
         r->xyz = std::move(dxyz);
+        {
+            // The pool keeps the visits' memory for the first run (up to what it keeps free).
+            PoolScope pool(s, false);
+            DevBuf<double> visits;
+            r->take_visits(&visits);
+        }
         FG_CUDA(cudaStreamSynchronize(s));
         *out = r.release();
     });
@@ -1348,6 +1362,13 @@ int femgpu_recovery_run_device(femgpu_recovery* r, const double* u, const double
     });
 }
 
+int femgpu_recovery_set_scratch(femgpu_recovery* r, size_t bytes) {
+    return recovery_guarded([&] {
+        need(r != nullptr, "a null handle");
+        r->visit_limit = bytes;
+    });
+}
+
 int femgpu_recovery_probes(femgpu_recovery* r, const double* u, const double* dtemp,
                            const double* temperature, size_t nprobes, const double* points,
                            const char* const* names, double* displacement, double* stress,
@@ -1411,7 +1432,7 @@ size_t femgpu_recovery_bytes(const femgpu_recovery* r) {
     if (!r) return 0;
     return r->t10.bytes() + r->rec.bytes() + r->mats.bytes() + r->singular.bytes() +
            r->hrec.bytes() + r->hmodes.bytes() + r->amp.bytes() +
-           r->place.bytes() + r->u4.bytes() + r->visits.bytes() + r->peak.bytes() + r->dpeaks.bytes() +
+           r->place.bytes() + r->u4.bytes() + r->peak.bytes() + r->dpeaks.bytes() +
            r->xyz.bytes() +
            r->inc.start.bytes() +
            r->inc.of_node.bytes() + r->du.bytes() + r->ddt.bytes() + r->dstress.bytes() +

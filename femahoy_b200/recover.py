@@ -121,6 +121,12 @@ class Recovery:
     def handle(self):
         return self._h
 
+    def with_scratch(self, bytes):
+        """The most device memory a run may take as scratch (tetrahedra; 4 GiB by default). With
+        less than 640 bytes per cell the points evaluate their own visits: the same bits, slower."""
+        L.check(L.lib().femgpu_recovery_set_scratch(self._h, bytes))
+        return self
+
     def run(self, u, dtemp=None, *, peaks=True, principal=True):
         """Host arrays in and out: a dict of stress (n, 6), strain (n, 6), mises (n,),
         principal (n, 3) or None, and peaks (a list of Peak, 1 per part) or None."""

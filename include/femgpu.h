@@ -710,6 +710,10 @@ int femgpu_recovery_run(femgpu_recovery* r, const double* u, const double* dtemp
 int femgpu_recovery_run_device(femgpu_recovery* r, const double* u, const double* dtemp,
                                double* stress, double* strain, double* mises, double* principal,
                                femgpu_peak* peaks);
+/* The most device memory that a recovery of tetrahedra may take as scratch while it runs (640
+ * bytes per cell, from the library's pool; 4 GiB by default). Where that is not enough, or the
+ * device has no room, the points evaluate their own visits: the same bits, about 1.7 times the time. */
+int femgpu_recovery_set_scratch(femgpu_recovery* r, size_t bytes);
 /* The probes of a P2 model (elastic_tet.rs:428-467): for each point (3 coordinates each), the
  * cells whose volume coordinates of the point are all >= -1e-9 (cells_at, elastic_tet.rs:538-553),
  * each taking the share 1 / hits of the displacement (the 10 functions of tet10.rs:51-60), the

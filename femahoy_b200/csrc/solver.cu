@@ -2008,13 +2008,21 @@ static void tile_attributes() {
 
 // Whether a finest FP32 stencil level (K = 8, large enough to fill the GPU with tiles) takes the
 // tile kernels: mode 2 yes, mode 1 no, mode 0 when its residual by tiles is faster than by the
-// kernel the autotuner chose (the same timing as tune_operator). A probe whose copies time out
-// keeps the direct kernels.
-static void tune_tiles(Operator<float>* op, int mode, cudaStream_t s) {
+// kernel the autotuner chose, kept per size class as the other choices are (`forced`: a kernel was
+// asked for, and keeps the level). A probe whose copies time out keeps the direct kernels.
+static void tune_tiles(Operator<float>* op, int mode, bool forced, cudaStream_t s) {
     op->bulk = false;
-    if (mode == 1 || !op->stencil || op->half || op->K != 8) return;
+    if (mode == 1 || (mode == 0 && forced) || !op->stencil || op->half || op->K != 8) return;
     int64_t n = op->n;
     if (n < (int64_t)STENCIL_TILE * NUM_SMS) return;
+    const int kernel = op->march ? 4 : op->pair ? 3 : op->unrolled ? 1 : 0;
+    const std::array<int64_t, 5> key{3, kernel, op->K, log2_of(n), 0};
+    int v = 0;
+    if (mode == 0 && tune_lookup(key, &v)) {
+        op->bulk = v != 0;
+        if (op->bulk) tile_attributes();
+        return;
+    }
     tile_attributes();
     DevBuf<float> x(n), b(n), r(n);
     x.zero(s);
@@ -2022,35 +2030,34 @@ static void tune_tiles(Operator<float>* op, int mode, cudaStream_t s) {
     DevBuf<int> done(1), timeout(1);
     done.zero(s);
     timeout.zero(s);
-    const StencilView<float> v = op->sview();
+    const StencilView<float> v0 = op->sview();
     auto probe = [&]() {
         k_stencil_tiles<8, false><<<tile_grid(n), BULK_TH, tile_smem<false>(), s>>>(
-            v, b.p, x.p, nullptr, 0.f, 0.f, nullptr, r.p, done.p, timeout.p, BULK_SPIN);
+            v0, b.p, x.p, nullptr, 0.f, 0.f, nullptr, r.p, done.p, timeout.p, BULK_SPIN);
     };
-    cudaEvent_t e0, e1;
-    FG_CUDA(cudaEventCreate(&e0));
-    FG_CUDA(cudaEventCreate(&e1));
-    for (int w = 0; w < 10; ++w) probe();
-    FG_CHECK_LAUNCH();
-    double best = 1e30;
-    for (int round = 0; round < 4; ++round) {
-        FG_CUDA(cudaEventRecord(e0, s));
-        for (int k = 0; k < 5; ++k) probe();
-        FG_CUDA(cudaEventRecord(e1, s));
-        FG_CUDA(cudaEventSynchronize(e1));
-        float ms = 0;
-        FG_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        best = std::min(best, (double)ms / 5);
+    op->probe_ms[2] = time_best(probe, 10, 4, s);
+    const bool late = fetch(timeout.p, s) != 0;
+    if (mode == 0) {
+        // The chosen kernel's own time, unless tune_operator has just taken it.
+        if (op->probe_ms[kernel] == 0.0)
+            op->probe_ms[kernel] = time_best(
+                [&] {
+                    if (op->march)
+                        launch_march<float, false>(false, *op, s, b.p, x.p, nullptr, 0.f, 0.f,
+                                                   nullptr, r.p, done.p);
+                    else if (op->pair)
+                        k_residual_pair<float, 8><<<row_blocks(pair_threads(n)), TH, 0, s>>>(
+                            v0, b.p, x.p, r.p, done.p);
+                    else
+                        with_op(*op, [&](auto o) {
+                            k_residual<float><<<row_blocks(n), TH, 0, s>>>(o, b.p, x.p, r.p,
+                                                                           done.p);
+                        });
+                },
+                10, 4, s);
+        tune_store(key, !late && op->probe_ms[2] < op->probe_ms[kernel]);
     }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    op->probe_ms[2] = best;
-    if (fetch(timeout.p, s)) return;
-    const double direct = op->march  ? op->probe_ms[4]
-                          : op->pair   ? op->probe_ms[3]
-                          : op->unrolled ? op->probe_ms[1]
-                                         : op->probe_ms[0];
-    op->bulk = mode == 2 || best < direct;
+    op->bulk = !late && (mode == 2 || op->probe_ms[2] < op->probe_ms[kernel]);
 }
 
 // lambda_max of D^-1 A by the power method in the D inner product (15 steps), on the device.
@@ -2180,14 +2187,15 @@ static std::string describe_op(const Operator<T>& op) {
         std::snprintf(buf, sizeof buf, "sell C=%d nnz=%lld", op.sell.C, (long long)op.nnz);
     } else {
         std::snprintf(buf, sizeof buf,
-                      "stencil K=%d %s%s (probe %.1f / %.1f / %.1f / %.1f us)%s nnz=%lld", op.K,
+                      "stencil K=%d %s%s (probe %.1f / %.1f / %.1f / %.1f us, tiles %.1f)%s nnz=%lld",
+                      op.K,
                       op.half ? "fp16 " : "",
                       op.march  ? "marching planes"
                       : op.pair ? "unrolled, 2 rows per thread"
                       : op.unrolled ? "unrolled"
                                     : "loop",
                       op.probe_ms[0] * 1e3, op.probe_ms[1] * 1e3, op.probe_ms[3] * 1e3,
-                      op.probe_ms[4] < 1e29 ? op.probe_ms[4] * 1e3 : 0.0,
+                      op.probe_ms[4] < 1e29 ? op.probe_ms[4] * 1e3 : 0.0, op.probe_ms[2] * 1e3,
                       op.bulk ? ", steps from bulk-copied tiles" : "", (long long)op.nnz);
     }
     return buf;
@@ -2586,7 +2594,7 @@ void SolverImpl::build_levels(const std::vector<const DevCsr*>& mats, std::vecto
             tune_operator(&lv.A, opt_.stencil, s_);
             if (!opt_.sell_c) tune_sell(d, &lv.A, s_);
             if constexpr (std::is_same<T, float>::value)
-                if (l == 0) tune_tiles(&lv.A, opt_.tiles, s_);
+                if (l == 0) tune_tiles(&lv.A, opt_.tiles, opt_.stencil > 0, s_);
         }
         std::optional<PhaseTimer> t_lam;
         t_lam.emplace(this, "diagonals and lambda_max", s_);

@@ -50,8 +50,9 @@ inline int blocks_for(int64_t n, int threads, int cap = NUM_SMS * 16) {
 //
 // What it is for: a model's way from the mesh to the solution makes and frees about 190 buffers,
 // each cudaMalloc and cudaFree mapping or unmapping memory (0.15 ms each, more when other
-// processes of the machine do the same): 60 of the 91 ms of a 64^3 heat model on B200, 38 of the
-// 60 ms of a 60 x 8 x 8 P2 beam.
+// processes of the machine do the same). With every buffer a cudaMalloc of its own a 64^3 heat
+// model takes 88 ms on B200 and a 60 x 8 x 8 P2 beam 55 (medians, quiet machine); with the pool 34
+// and 25.
 //
 // The rules that keep it safe. A scope is opened only around code whose buffers are used on the
 // scope's stream alone until it has been synchronized, and every buffer that outlives the scope

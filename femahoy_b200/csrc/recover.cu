@@ -18,7 +18,8 @@
 // The visits are evaluated cell by cell (a thread takes 10 or 2 of a cell, with its record, points
 // and displacements in registers), leaving strain, dt and material in 64 bytes each; then a thread
 // per point gathers its visits' 64 bytes and forms their stresses and the means. What bounds it:
-// the FP64 operations of the visits (about 300 each) and the visits' 64 bytes written and read.
+// the latency of the visits' FP64 chains and loads; a thread's 164 registers leave 17 % of the
+// warps active (SM 46 %, DRAM 22 % of their peaks in the visits' kernel).
 // With a thread per point evaluating its own visits, the lanes of a warp sat in different cells,
 // so each load of a record, a point number or a displacement touched up to 32 lines and the L1
 // set the time: 531 us for the 160 x 20 x 20 P2 beam (384,000 cells, 3.84M visits; the 3 largest
@@ -406,8 +407,12 @@ __device__ __forceinline__ void write_point(int64_t v, int64_t count, double ss[
 
 // The most that the visits' 64 bytes may take unless the caller sets it.
 constexpr size_t VISIT_BYTES_MAX = (size_t)4 << 30;
-// From this many cells on a thread takes all 10 visits of a cell.
-constexpr int64_t WHOLE_CELLS = 100'000;
+// From this many cells on a thread takes all 10 visits of a cell: the cell's record and
+// displacements are then loaded once; below, 5 threads per cell fill the device better. A recovery's
+// kernels with 2 / 10 visits per thread (us, 4 parts with peaks): 7,680 cells 44 / 47, 14,580 cells
+// 50 / 47, 36,300 cells 64 / 53, 98,280 cells 111 / 88, 384,000 cells 283 / 238. (5 visits: 45 at
+// 14,580 cells, 88 at 98,280, 252 at 384,000: not worth a third form.)
+constexpr int64_t WHOLE_CELLS = 12'000;
 constexpr int VISIT_BLOCKS = 8;  // blocks per SM
 
 // A 32-byte store; p is 32-byte aligned.

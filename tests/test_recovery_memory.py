@@ -22,8 +22,10 @@ def _same(a, b):
 
 
 @pytest.mark.parametrize("dims,nparts", [((1, 1, 1), 1), ((7, 5, 3), 3), ((12, 9, 8), 70),
+                                         ((19, 15, 7), 2), ((20, 10, 10), 3),
                                          ((34, 23, 22), 5)])
 def test_points_that_evaluate_their_own_visits_give_the_same_bits(dims, nparts):
+    """6 to 103,224 cells, with 11,970 and 12,000 at the line of 10 visits per thread."""
     c = random_case(dims, nparts=nparts)
     r = _new(c, nparts)
     for dtemp in (None, c["dtemp"]):

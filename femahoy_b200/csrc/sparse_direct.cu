@@ -156,7 +156,8 @@ __global__ void __launch_bounds__(TH)
 // mesh 1,633 -> 393 -> 199 us, its kernels timed one by one (the early trigger takes 52 us more
 // off each iteration of that solve: 22.9 -> 21.0 ms). Before, 1 block took a whole supernode and
 // the large ones near the root left the other SMs idle. The error of 1 application against
-// extended precision stayed: 1e-12 to 6e-11 on P2 beams of 14,580 to 37,440 unknowns on any form.
+// extended precision is 1e-12 to 6e-11 on P2 beams of 14,580 to 37,440 unknowns on any form, and its
+// residual that of the substitution (k_large_panel).
 constexpr int SOLVE_WARPS = 16;
 constexpr int SOLVE_TH = 32 * SOLVE_WARPS;
 constexpr int ZCAP = 128;  // right side values staged per warp of a task

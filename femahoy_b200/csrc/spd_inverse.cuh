@@ -18,9 +18,11 @@
 // 0.85 ms (25 Tflop/s): 4.5 ms. By panels of 32 columns with W formed afterwards the inverse of
 // the 128^3 heat cube's 4,913 unknowns took 23 ms, of which 0.8 us per column went to the panels'
 // diagonal blocks alone, and every rank-32 update read and wrote the whole trailing matrix. The
-// products sum 128 terms before they meet the matrix, so it rounds no more often than before:
-// 1 product with the inverse of P1 cantilevers of 3,000 to 3,900 unknowns is 7e-13 to 4.3e-11 off
-// an extended precision solution (0.9e-12 to 4.9e-11 before).
+// products sum 128 terms before they meet the matrix, so it rounds no more often than before. 1
+// product with the inverse of 18 P1 cantilevers of 1,380 to 2,700 unknowns (3 right sides each, off
+// an extended precision solution, geometric means; before in brackets): Poisson ratios of 0.25 to
+// 0.35 1.9e-12 (2.9e-12), stiffness jumps of 1e6 7.9e-12 (8.5e-12), a ratio of 0.4999 1.4e-10
+// (0.8e-10; a Cholesky factor with substitutions on the host 4.1e-10).
 #pragma once
 #include <cstdint>
 

@@ -165,9 +165,9 @@ void figures(const Ordered& o, const std::vector<int64_t>& first, uint64_t* entr
 // while the zeros that its panel then stores stay a small share of it, a larger one for narrow
 // panels. The columns keep their order, so the factor's pivots are the same; the panels grow
 // a little and the tree loses levels, each of which costs a solve 2 launches and the latency of
-// the level before. On the 50 x 5 x 5 P2 beam: 3,039 -> 947 supernodes, 23 -> 11 levels, panels
-// 15.6M -> 16.5M values, fronts 134M -> 91M; a 32^3 heat cube 73 -> 11 levels, 11.5M -> 13.0M. A
-// share of 0.2 stores a quarter more for 1 level less.
+// the level before. On the 50 x 5 x 5 P2 beam (36,300 unknowns): 2,872 -> 979 supernodes, 22 -> 11
+// levels, panels 15.0M -> 16.3M values, fronts 128M -> 90M; a 32^3 heat cube 73 -> 11 levels, 11.0M
+// -> 13.0M. A share of 0.2 stores a quarter more for 1 level less.
 constexpr int64_t NARROW = 32;
 constexpr double SHARE_NARROW = 0.5, SHARE = 0.1;
 

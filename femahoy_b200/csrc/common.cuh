@@ -22,14 +22,18 @@ struct Failure : std::runtime_error {
 
 void set_last_error(const std::string& s);
 
+// The runtime keeps a failed call's error for the next cudaGetLastError, which would then blame a
+// later launch that is fine: it is taken out here.
 #define FG_CUDA(call)                                                                  \
     do {                                                                               \
         cudaError_t e_ = (call);                                                       \
-        if (e_ != cudaSuccess)                                                         \
+        if (e_ != cudaSuccess) {                                                       \
+            cudaGetLastError();                                                        \
             throw ::femgpu::Failure(FEMGPU_ERR_CUDA, std::string("CUDA error: ") +    \
                                                          cudaGetErrorString(e_) +     \
                                                          " at " __FILE__ ":" +        \
                                                          std::to_string(__LINE__));   \
+        }                                                                              \
     } while (0)
 
 #define FG_CHECK_LAUNCH() FG_CUDA(cudaGetLastError())

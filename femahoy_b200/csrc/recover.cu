@@ -1001,7 +1001,6 @@ struct femgpu_recovery {
             v->alloc(80 * (size_t)nel);
         } catch (const Failure&) {  // no room: the points evaluate their own visits
             v->release();
-            cudaGetLastError();
         }
     }
 

@@ -64,3 +64,26 @@ def test_trim_gives_the_free_memory_back():
     assert start - _free() >= GIB // 2  # kept for the next setup
     fg.trim()
     assert start - _free() <= GIB // 16
+
+
+def test_a_refused_allocation_leaves_no_error_behind():
+    """A call that finds no memory fails by itself; the next one, with room again, is answered."""
+    torch = pytest.importorskip("torch")
+    h = mg.heat_cube(64)
+    k = fg.Csr.assemble(fg.P1_HEAT, h.xyz, h.nodes, h.coef)
+    rows = np.arange(k.shape[0])
+    x = np.ones(k.shape[0])
+    want = k.mul(x)
+    k.submatrix(rows)
+    gc.collect()
+    fg.trim()
+    torch.cuda.empty_cache()
+    hold = torch.empty(_free() - (24 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        with pytest.raises(fg.FemError, match="out of memory"):
+            k.submatrix(rows)
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+    assert np.array_equal(k.mul(x), want)
+    assert k.submatrix(rows).shape == k.shape

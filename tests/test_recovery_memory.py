@@ -64,3 +64,20 @@ def test_scratch_leaves_room_for_the_outputs():
     finally:
         del hold
         torch.cuda.empty_cache()
+
+
+def test_threads_side_by_side_give_the_same_bits():
+    """Each run takes its scratch from the pool that all of them share."""
+    from concurrent.futures import ThreadPoolExecutor
+    cases = [random_case(d, nparts=2) for d in ((9, 7, 5), (20, 10, 10), (14, 9, 8), (24, 11, 9))]
+    made = [_new(c, 2) for c in cases]
+    alone = [r.run(c["u"], c["dtemp"]) for r, c in zip(made, cases)]
+
+    def again(k):
+        return [made[k].run(cases[k]["u"], cases[k]["dtemp"]) for _ in range(6)]
+
+    with ThreadPoolExecutor(max_workers=len(made)) as pool:
+        for want, runs in zip(alone, pool.map(again, range(len(made)))):
+            for got in runs:
+                for k in ("stress", "strain", "mises", "principal"):
+                    assert _same(got[k], want[k]), k
